@@ -45,6 +45,14 @@ struct curfpContext {
 
 namespace rfp {
 
+// What the tile Cholesky (k_chol.cuh) takes in one launch: a diagonal block
+// of up to kCholRows, with up to kCholPanelRows rows below it, and a whole RFP
+// matrix of up to kCholRfpRows when its trailing update is too small for the
+// tensor cores (FP64: always).  Above, the recursion's larger products win.
+constexpr int kCholRows = 2048;
+constexpr int kCholPanelRows = 2048;
+constexpr int kCholRfpRows = 4096;
+
 // The CUDA executor for FP32 (SIMT and split-BF16 tensor-core contractions)
 // and FP64 (SIMT DFMA) element types.
 template <typename T>
@@ -54,11 +62,10 @@ class CudaExecT : public ExecT<T> {
       : ctx_(ctx), abort_(abort_flag) {}
   int gemm(const GemmProbT<T>* p, int count) override;
   int potrf_tile(ViewT<T> L, int n, int info_base) override;
-  // 128-row tiles.  (A 256-row FP32 tile, one CTA of 512 threads, measured
-  // 157 us per tile against 2 x 57 us for two 128-row tiles: it moves the
-  // 128^3 trailing update of the level above from a multi-CTA SYRK into one
-  // CTA.)
-  int potrf_tile_rows() const override { return kPotrfTile; }
+  int potrf_tile_rows() const override { return kCholRows; }
+  int potrf_blocks(ViewT<T> V11, ViewT<T> V21, ViewT<T> V22, int n1, int n2) override;
+  bool has_panel(int n1, int n2) const override;
+  int potrf_panel(ViewT<T> L, ViewT<T> A21, int n1, int n2, int info_base) override;
   int trtri_blocks(ViewT<T> L, int n, int nb, T* W) override;
   int trtri_tile(ViewT<T> L, int n) override;
   int lauum_tile(ViewT<T> L, int n) override;

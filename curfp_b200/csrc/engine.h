@@ -90,6 +90,23 @@ class ExecT {
   // Largest diagonal tile potrf_tile takes (a multiple of kPotrfTile); the
   // recursive Cholesky splits down to it.
   virtual int potrf_tile_rows() const { return kPotrfTile; }
+  // In-place Cholesky of the matrix given by its logical lower blocks (V11
+  // n1 x n1, V21 n2 x n1, V22 n2 x n2) as one operation, info as for
+  // potrf_tile with base 0, or kNotSupported.
+  virtual int potrf_blocks(ViewT<T> V11, ViewT<T> V21, ViewT<T> V22, int n1, int n2) {
+    (void)V11; (void)V21; (void)V22; (void)n1; (void)n2;
+    return kNotSupported;
+  }
+  // In-place Cholesky of L (n1 x n1) and A21 := A21 L^-T (n2 x n1) as one
+  // operation, for the sizes has_panel() names.
+  virtual bool has_panel(int n1, int n2) const {
+    (void)n1; (void)n2;
+    return false;
+  }
+  virtual int potrf_panel(ViewT<T> L, ViewT<T> A21, int n1, int n2, int info_base) {
+    (void)L; (void)A21; (void)n1; (void)n2; (void)info_base;
+    return kNotSupported;
+  }
   // Called by the RFP factorization once the first diagonal block's work is
   // enqueued and before any work that reads the other blocks: an executor
   // may order that work after data it is still bringing in.

@@ -5,6 +5,7 @@
 #include <type_traits>
 
 #include "context.h"
+#include "k_chol.cuh"
 #include "k_gemm.cuh"
 #include "gemm_route.h"
 #include "k_skinny.cuh"
@@ -283,13 +284,36 @@ int CudaExecT<T>::potrf_adj_tile(ViewT<T> L, ViewT<T> G, int n) {
 }
 
 namespace {
-template <typename T, int NT, int THR>
-int launch_potrf(curfpContext* ctx, ViewT<T> L, int n, int info_base) {
-  constexpr int smem = ktile::potrf_smem<T, NT>();
-  static const bool attr = smem_attr(ktile::potrf_tile<T, NT, THR>, smem);
+// The tile Cholesky (k_chol.cuh) of the logical lower blocks V11, V21, V22,
+// or with panel set of V11 and V21 alone.
+template <typename T>
+int launch_chol(curfpContext* ctx, ViewT<T> V11, ViewT<T> V21, ViewT<T> V22, int n1, int n2,
+                bool panel, int info_base) {
+  kchol::Args<T> a{};
+  a.v11 = V11; a.v21 = V21; a.v22 = V22;
+  a.n1 = n1; a.n2 = n2;
+  a.nb1 = (n1 + kchol::NB - 1) / kchol::NB;
+  a.nb = a.nb1 + (n2 + kchol::NB - 1) / kchol::NB;
+  a.nbf = panel ? a.nb1 : a.nb;
+  const size_t tiles = (size_t)kchol::tile_count(a.nb, a.nbf), words = 1 + tiles;
+  a.ws = static_cast<T*>(
+      grow_buffer(ctx, &ctx->ws, &ctx->ws_bytes, tiles * kchol::TILE * sizeof(T)));
+  a.sync = static_cast<int*>(grow_buffer(ctx, &ctx->tsv, &ctx->tsv_bytes, words * sizeof(int)));
+  if (!a.ws || !a.sync) return 2;
+  if (cudaMemsetAsync(a.sync, 0, words * sizeof(int), ctx->stream) != cudaSuccess) return 4;
+  a.info = ctx->d_info;
+  a.err = ctx->d_info + 1;
+  a.info_base = info_base;
+  constexpr int smem = kchol::smem_bytes<T>();
+  static const bool attr = smem_attr(kchol::chol_wave<T>, smem);
   if (!attr) return 4;
-  ktile::potrf_tile<T, NT, THR><<<1, THR, smem, ctx->stream>>>(L, n, info_base, ctx->d_info);
+  const double n = (double)n1 + n2, m = panel ? n2 : 0;
+  ProfScope ps(ctx->prof, ctx->stream, K_POTRF,
+               panel ? (n1 / 3.0 + m) * n1 * n1 : n * n * n / 3.0, 0);
+  ps.shape(n1, n2, panel ? 1 : 0, (int)tiles);
+  kchol::chol_wave<T><<<kchol::cta_count(a.nb, a.nbf), kchol::threads<T>(), smem, ctx->stream>>>(a);
   ++ctx->launches;
+  ++ctx->wait_launches;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 }  // namespace
@@ -298,8 +322,25 @@ template <typename T>
 int CudaExecT<T>::potrf_tile(ViewT<T> L, int n, int info_base) {
   if (n <= 0) return 0;
   if (n > potrf_tile_rows()) return 3;
-  ProfScope ps(ctx_->prof, ctx_->stream, K_POTRF, (double)n * n * n / 3.0, 0);
-  return launch_potrf<T, ktile::PT, 256>(ctx_, L, n, info_base);
+  return launch_chol<T>(ctx_, L, L, L, n, 0, false, info_base);
+}
+
+template <typename T>
+int CudaExecT<T>::potrf_blocks(ViewT<T> V11, ViewT<T> V21, ViewT<T> V22, int n1, int n2) {
+  if (n1 + n2 > kCholRfpRows || (sizeof(T) == 4 && tc_worthwhile(n2, n2, n1)))
+    return kNotSupported;
+  const int rc = after_first_block();
+  return rc ? rc : launch_chol<T>(ctx_, V11, V21, V22, n1, n2, false, 0);
+}
+
+template <typename T>
+bool CudaExecT<T>::has_panel(int n1, int n2) const {
+  return n1 > 0 && n2 > 0 && n1 <= potrf_tile_rows() && n2 <= kCholPanelRows;
+}
+
+template <typename T>
+int CudaExecT<T>::potrf_panel(ViewT<T> L, ViewT<T> A21, int n1, int n2, int info_base) {
+  return launch_chol<T>(ctx_, L, A21, A21, n1, n2, true, info_base);
 }
 
 template <typename T>

@@ -1,0 +1,674 @@
+// k_chol.cuh — tile Cholesky of a lower-triangular matrix, with the rows below
+// it, in one launch.
+//
+// The matrix is cut into 64 x 64 tiles that hand their results on through
+// flags in L2, so the time is the chain of diagonal tiles.  (A recursion down
+// to single-CTA 128-row tiles instead pays a chain of small launches: tile,
+// inverses, solve, update, ~100 us per 128 columns.)
+//
+// Tickets (atomic counter) go out in the order: the first diagonal tile, then
+// for each tile column c the tiles (c+1, c), (c+2, c), ...  A CTA waits only
+// on smaller tickets, which are running or done, so no co-residency is needed
+// and the scheme cannot deadlock.  CTA (i, c):
+//   acc  = sum_{k<c} L_ik L_ck^T as the tiles are published,
+//   X    = L_ic = (A_ic - acc) W_c^T once W_c = inv(L_cc) is published;
+// and, when i = c + 1, it also factors the next diagonal tile,
+//   S    = A_ii - sum_{k<c} L_ik L_ik^T - X X^T = L_ii L_ii^T,  W_i = inv(L_ii).
+//
+// The sums run on 8 x 8 register tiles: shared memory returns 128 bytes a
+// cycle, so a 4 x 4 tile (8 loads for 16 FMAs) would run at half the FMA rate
+// and 8 x 8 is where the two meet.  64 threads cover a tile; the CTA's groups
+// of 64 threads split k and their partial sums meet once per CTA.  In a
+// diagonal CTA half of the groups sum for X and half for S.
+//
+// The chain from one W to the next is ordered so that only what the next
+// pivot needs is on it: X's upper 32 rows, S's upper-left quarter, its factor
+// by warp 0 (factor32); meanwhile warp 1 follows column by column with the
+// quarter's inverse and a further set of warps forms X's lower rows and the
+// rest of S.
+//
+// Published tiles live in a packed workspace (k-major 64 x 64, element (a, b)
+// at b * 64 + a), whatever the matrix's strides: consumers fetch them by
+// 16-byte L2-only cp.async (cp.async.cg), and the matrix itself is read and
+// written once, by the tile's owner.  Partial tiles are padded with the
+// identity.
+//
+// The matrix is given as the logical lower blocks V11 (n1 x n1), V21
+// (n2 x n1) and V22 (n2 x n2) of an RFP array.  The first nbf tile columns
+// are factored: all of them, or only the first block's (then V21 becomes
+// V21 L11^-T and V22 is not touched; a plain matrix has n2 = 0).
+// Bound by the chain: a 64-column step takes 13.5 us in FP32 and 23.6 us in
+// FP64 (n = 2000; about 5 us of it the two 32-column factors), against ~50 us
+// per 64 columns of the recursion with 128-row tiles.  RFP factorizations on
+// B200, recursion -> this: n = 250 0.19 -> 0.060 ms, n = 4095 4.3 -> 1.14 ms
+// (with one tensor-core update), FP64 n = 3000 4.8 -> 1.2 ms.
+// Waits are bounded; a CTA that gives up (or whose diagonal tile has a
+// non-positive pivot) publishes poisoned flags so that its dependents stop.
+#pragma once
+#include <climits>
+#include <cstdint>
+
+#include "engine.h"
+#include "k_tile.cuh"
+#include "k_trsv.cuh"
+
+namespace rfp {
+namespace kchol {
+
+constexpr int NB = 64;
+constexpr int TILE = NB * NB;
+constexpr int LDW = NB + 4;  // column stride of W in shared memory (conflict-free 16-byte columns)
+
+// 64 threads per group; FP32 has 512 threads, FP64 256 (registers).
+template <typename T> constexpr int threads() { return sizeof(T) == 4 ? 512 : 256; }
+template <typename T> constexpr int groups() { return threads<T>() / 64; }
+// two double-buffered operand tiles, T, S, W
+template <typename T> constexpr int smem_bytes() { return (6 * TILE + NB * LDW) * (int)sizeof(T); }
+
+template <typename T>
+struct Args {
+  ViewT<T> v11, v21, v22;
+  int n1, n2, nb1, nb;  // orders, tiles of the first block, tiles in all
+  int nbf;              // tile columns factored: nb, or nb1
+  T* ws;                // published tiles (tile_index; W_i at (i, i))
+  int* sync;            // [0] ticket, [1 + tile] flags (0 not ready, 1 ready, -1 poisoned)
+  int* info;            // pivot failures (INT_MAX: none)
+  int* err;             // wait timeouts
+  int info_base;
+};
+
+// Index of published tile (i, k): packed lower triangle, then full rows of
+// nbf tiles below the factored columns.
+__host__ __device__ __forceinline__ int tile_index(int nbf, int i, int k) {
+  return i < nbf ? i * (i + 1) / 2 + k : nbf * (nbf + 1) / 2 + (i - nbf) * nbf + k;
+}
+inline int64_t tile_count(int nb, int nbf) {
+  return (int64_t)nbf * (nbf + 1) / 2 + (int64_t)(nb - nbf) * nbf;
+}
+// CTAs of a launch: the first diagonal tile and the tiles below the diagonal
+// of the factored columns.
+inline int cta_count(int nb, int nbf) {
+  int t = 1;
+  for (int c = 0; c < nbf; ++c) t += nb - 1 - c;
+  return t;
+}
+
+// 16 bytes by cp.async, L2 only (the data was written by CTAs of this launch).
+__device__ __forceinline__ void cp16(void* smem, const void* g) {
+  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(g) : "memory");
+}
+template <typename T>
+__device__ __forceinline__ void fetch_tile(T* s, const T* g) {
+  constexpr int VW = 16 / (int)sizeof(T);
+#pragma unroll
+  for (int u = 0; u < TILE / VW / threads<T>(); ++u) {
+    const int e = (threadIdx.x + threads<T>() * u) * VW;
+    cp16(s + e, g + e);
+  }
+}
+template <int ID, int COUNT>
+__device__ __forceinline__ void bar_sync() {
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(COUNT) : "memory");
+}
+template <int COUNT>
+__device__ __forceinline__ void bar_sync_id(int id) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(COUNT) : "memory");
+}
+template <int COUNT>
+__device__ __forceinline__ void bar_arrive_id(int id) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(COUNT) : "memory");
+}
+
+using ktrsv::lds4;
+__device__ __forceinline__ void sts4(float* p, const float (&v)[4]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void sts4(double* p, const double (&v)[4]) {
+  reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
+  reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
+}
+
+// acc += A B^T over k in [k0, k0 + KG), A and B k-major (column stride 64);
+// thread u of 64: rows 4 (u % 8) + {0, 32}.., columns 4 (u / 8) + {0, 32}..
+template <int KG, typename T>
+__device__ __forceinline__ void product8(T (&acc)[8][8], const T* A, const T* B, int k0, int u) {
+  const T* a0 = A + k0 * NB + (u & 7) * 4;
+  const T* b0 = B + k0 * NB + (u >> 3) * 4;
+#pragma unroll 4
+  for (int k = 0; k < KG; ++k) {
+    T a[8], b[8];
+    lds4(a0 + k * NB, *reinterpret_cast<T(*)[4]>(a));
+    lds4(a0 + k * NB + 32, *reinterpret_cast<T(*)[4]>(a + 4));
+    lds4(b0 + k * NB, *reinterpret_cast<T(*)[4]>(b));
+    lds4(b0 + k * NB + 32, *reinterpret_cast<T(*)[4]>(b + 4));
+#pragma unroll
+    for (int p = 0; p < 8; ++p)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[p][q] = fma(a[p], b[q], acc[p][q]);
+  }
+}
+template <typename T>
+__device__ __forceinline__ void store8(T* s, const T (&acc)[8][8], int u) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const T v[4] = {acc[4 * h][q], acc[4 * h + 1][q], acc[4 * h + 2][q], acc[4 * h + 3][q]};
+      sts4(s + ((u >> 3) * 4 + (q >> 2) * 32 + (q & 3)) * NB + (u & 7) * 4 + 32 * h, v);
+    }
+}
+template <typename T>
+__device__ __forceinline__ void add8(T (&acc)[8][8], const T* s, int u) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      T v[4];
+      lds4(s + ((u >> 3) * 4 + (q >> 2) * 32 + (q & 3)) * NB + (u & 7) * 4 + 32 * h, v);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[4 * h + e][q] += v[e];
+    }
+}
+// dst -= the sum of N partial tiles at src, src + TILE, ... (all threads).
+template <int N, typename T>
+__device__ __forceinline__ void subtract(T* dst, const T* src) {
+#pragma unroll
+  for (int w = 0; w < TILE / 4 / threads<T>(); ++w) {
+    const int e = (threadIdx.x + threads<T>() * w) * 4;
+    T s[4], v[4];
+    lds4(src + e, s);
+#pragma unroll
+    for (int i = 1; i < N; ++i) {
+      lds4(src + i * TILE + e, v);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) s[q] += v[q];
+    }
+    lds4(dst + e, v);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] -= s[q];
+    sts4(dst + e, v);
+  }
+}
+
+// out(4 x 4 at rows 4 tr, columns 4 tc) = sum_{k0 <= k < k1} A B^T, column
+// strides LDA, LDB.
+template <int LDA, int LDB, typename T>
+__device__ __forceinline__ void product4(T (&o)[4][4], const T* A, const T* B, int k0, int k1,
+                                         int tr, int tc) {
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) o[p][q] = T(0);
+#pragma unroll 4
+  for (int k = k0; k < k1; ++k) {
+    T a[4], b[4];
+    lds4(A + k * LDA + tr * 4, a);
+    lds4(B + k * LDB + tc * 4, b);
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) o[p][q] = fma(a[p], b[q], o[p][q]);
+  }
+}
+// The sum over G groups of CNT threads each (thread u of group g; COUNT =
+// G * CNT threads meet at barrier ID) into group 0; red: (G - 1) * CNT * 16.
+template <int G, int CNT, int ID, typename T>
+__device__ __forceinline__ void reduce4(T (&o)[4][4], T* red, int g, int u) {
+  if constexpr (G > 1) {
+    if (g > 0) {
+#pragma unroll
+      for (int p = 0; p < 4; ++p) sts4(red + (((g - 1) * 4 + p) * CNT + u) * 4, o[p]);
+    }
+    bar_sync<ID, G * CNT>();
+    if (g == 0) {
+#pragma unroll
+      for (int i = 0; i < G - 1; ++i)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          T v[4];
+          lds4(red + ((i * 4 + p) * CNT + u) * 4, v);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) o[p][q] += v[q];
+        }
+    }
+  }
+}
+// s(rows 4 tr.., columns 4 tc..; column stride LD) = o, or -= o.
+template <int LD, bool kSub, typename T>
+__device__ __forceinline__ void put4(T* s, const T (&o)[4][4], int tr, int tc) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    T* p = s + (tc * 4 + q) * LD + tr * 4;
+    T v[4] = {o[0][q], o[1][q], o[2][q], o[3][q]};
+    if (kSub) {
+      T w[4];
+      lds4(p, w);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = w[e] - v[e];
+    }
+    sts4(p, v);
+  }
+}
+
+// 1/sqrt(d): the hardware estimate r and one Newton step for y = x^-1/2 in
+// the form r + r/2 (1 - d r^2), whose last rounding dominates its error.
+__device__ __forceinline__ float rsqrt_newton(float d) {
+  const float r = rsqrtf(d);
+  return fmaf(0.5f * r, fmaf(-d * r, r, 1.0f), r);
+}
+__device__ __forceinline__ double rsqrt_newton(double d) {
+  const double r = rsqrt(d);
+  return fma(0.5 * r, fma(-d * r, r, 1.0), r);
+}
+
+// One warp, lane = row: Cholesky factor of a 32 x 32 block s (column-major,
+// stride 64; lower triangle read, overwritten by the factor; garbage above
+// the diagonal).  The chain of a column is: update the next column, its pivot
+// by shuffle, rsqrt, scale.  The column goes to raw (32 x 32, column-major)
+// unscaled: it comes back as 16-byte broadcast reads behind the rsqrt, and
+// drives the inverse in another warp, which is let on every 8 columns
+// (barriers bar0 .. bar0 + 3).  After a failed pivot the remaining columns of
+// raw are not written, but all barriers are passed.  Returns 0, or 1 + the
+// failing column.
+template <typename T>
+__device__ __forceinline__ int factor32(T* s, T* raw, int bar0) {
+  const int lane = threadIdx.x & 31;
+  T a[32];
+#pragma unroll
+  for (int k = 0; k < 32; ++k) a[k] = s[k * NB + lane];
+  int fail = 0;
+  raw[lane] = a[0];
+  T d = __shfl_sync(0xffffffffu, a[0], 0);
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    if (!fail && !(d > T(0))) fail = j + 1;  // the same value in every lane
+    if (!fail) {
+      const T r = rsqrt_newton(d);
+      T lk[32];
+#pragma unroll
+      for (int v4 = (j + 1) / 4; v4 < 8; ++v4)
+        lds4(raw + j * 32 + 4 * v4, *reinterpret_cast<T(*)[4]>(lk + 4 * v4));
+      const T l = a[j] * r, t = l * r, dj = d;
+      if (j + 1 < 32) {
+        a[j + 1] = fma(-t, lk[j + 1], a[j + 1]);
+        d = __shfl_sync(0xffffffffu, a[j + 1], j + 1);
+        raw[(j + 1) * 32 + lane] = a[j + 1];
+        __syncwarp();
+      }
+      // the diagonal element: sqrt(d) = d r corrected by its residual
+      a[j] = lane == j ? fma(T(0.5) * r, fma(-l, l, dj), l) : l;
+#pragma unroll
+      for (int k = j + 2; k < 32; ++k) a[k] = fma(-t, lk[k], a[k]);
+    }
+    if ((j & 7) == 7) bar_arrive_id<64>(bar0 + (j >> 3));
+  }
+#pragma unroll
+  for (int k = 0; k < 32; ++k) s[k * NB + lane] = a[k];
+  return fail;
+}
+// The warp that follows factor32: lane = column of the inverse, written to w
+// (column-major, stride LDW, zeros above the diagonal).  Column j of the
+// factor is raw_j / sqrt(d_j), so x_j /= sqrt(d_j), then
+// x_i -= raw_ij (x_j / sqrt(d_j)).
+template <typename T>
+__device__ __forceinline__ void inverse32(T* w, const T* raw, int bar0) {
+  const int lane = threadIdx.x & 31;
+  T x[32];
+#pragma unroll
+  for (int k = 0; k < 32; ++k) x[k] = k == lane ? T(1) : T(0);
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    if ((j & 7) == 0) bar_sync_id<64>(bar0 + (j >> 3));
+    T lk[32];
+#pragma unroll
+    for (int v4 = j / 4; v4 < 8; ++v4)
+      lds4(raw + j * 32 + 4 * v4, *reinterpret_cast<T(*)[4]>(lk + 4 * v4));
+    const T r = rsqrt_newton(lk[j]);
+    const T u = x[j] * r, v = u * r;
+    x[j] = u;
+#pragma unroll
+    for (int k = j + 1; k < 32; ++k) x[k] = fma(-v, lk[k], x[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < 32; k += 4) {
+    const T v[4] = {x[k], x[k + 1], x[k + 2], x[k + 3]};
+    sts4(w + lane * LDW + k, v);
+  }
+}
+
+// Tile (row tile i, column tile j) of the matrix as a view and its extents.
+template <typename T>
+__device__ __forceinline__ ViewT<T> tile_view(const Args<T>& g, int i, int j, int& rows,
+                                              int& cols) {
+  const bool r2 = i >= g.nb1, c2 = j >= g.nb1;
+  const int li = (r2 ? i - g.nb1 : i) * NB, lj = (c2 ? j - g.nb1 : j) * NB;
+  rows = min(NB, (r2 ? g.n2 : g.n1) - li);
+  cols = min(NB, (c2 ? g.n2 : g.n1) - lj);
+  return sub(c2 ? g.v22 : (r2 ? g.v21 : g.v11), li, lj);
+}
+
+// Matrix tile -> k-major shared tile, zeros (diag: identity) outside; of a
+// diagonal tile only the lower triangle is read and zeros stand above it.
+template <typename T>
+__device__ __forceinline__ void load_matrix(T* s, ViewT<T> v, int rows, int cols, bool diag) {
+  const bool rowcont = (v.cs == 1 || v.cs == -1) && !(v.rs == 1 || v.rs == -1);
+#pragma unroll 4
+  for (int u = 0; u < TILE / threads<T>(); ++u) {
+    const int e = threadIdx.x + threads<T>() * u;
+    const int a = rowcont ? e / NB : e % NB, b = rowcont ? e % NB : e / NB;
+    T x = diag && a == b ? T(1) : T(0);
+    if (a < rows && b < cols && (!diag || a >= b))
+      x = __ldcg(v.p + (int64_t)a * v.rs + (int64_t)b * v.cs);
+    s[b * NB + a] = x;
+  }
+}
+template <typename T>
+__device__ __forceinline__ void store_matrix(const T* s, ViewT<T> v, int rows, int cols,
+                                             bool diag) {
+  const bool rowcont = (v.cs == 1 || v.cs == -1) && !(v.rs == 1 || v.rs == -1);
+#pragma unroll 4
+  for (int u = 0; u < TILE / threads<T>(); ++u) {
+    const int e = threadIdx.x + threads<T>() * u;
+    const int a = rowcont ? e / NB : e % NB, b = rowcont ? e % NB : e / NB;
+    if (a < rows && b < cols && (!diag || a >= b))
+      v.p[(int64_t)a * v.rs + (int64_t)b * v.cs] = s[b * NB + a];
+  }
+}
+
+// Both flags ready: 1; either poisoned: -1; else 0.
+__device__ __forceinline__ int peek2(const int* f, const int* g) {
+  const int a = ktrsv::ld_acquire(f), b = ktrsv::ld_acquire(g);
+  return a < 0 || b < 0 ? -1 : (a > 0 && b > 0 ? 1 : 0);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
+  if (g.info && *g.info != INT_MAX) return;
+  extern __shared__ __align__(16) unsigned char chol_raw[];
+  T* A0 = reinterpret_cast<T*>(chol_raw);  // L_ik, double-buffered
+  T* B0 = A0 + 2 * TILE;                   // L_ck, double-buffered
+  T* Ts = B0 + 2 * TILE;
+  T* Ss = Ts + TILE;
+  T* Ws = Ss + TILE;  // W_i, column stride LDW
+  __shared__ int sh_ticket, sh_ready[2], sh_state, sh_fail;
+  constexpr int THR = threads<T>(), G = groups<T>();
+  const int tid = threadIdx.x, grp = tid >> 6, u = tid & 63;
+  const int warp = tid >> 5, lane = tid & 31;
+  constexpr int NW = THR / 32;
+  if (tid == 0) {
+    sh_ticket = atomicAdd(g.sync, 1);
+    sh_fail = 0;
+  }
+  __syncthreads();
+  int* flags = g.sync + 1;
+  auto tidx = [&](int r, int k) { return tile_index(g.nbf, r, k); };
+  // ticket 0: diagonal tile 0; then column by column (c+1, c), (c+2, c), ...
+  int c = -1, i = 0;
+  if (sh_ticket > 0) {
+    int rem = sh_ticket - 1;
+    c = 0;
+    while (rem >= g.nb - 1 - c) rem -= g.nb - 1 - c++;
+    i = c + 1 + rem;
+  }
+  const bool diag = i == c + 1 && i < g.nbf;
+
+  int xr = 0, xc = 0, sr = 0, scols = 0;
+  ViewT<T> xv{}, sv{};
+  if (c >= 0) {
+    xv = tile_view(g, i, c, xr, xc);
+    load_matrix(Ts, xv, xr, xc, false);
+  }
+  if (diag) {
+    sv = tile_view(g, i, i, sr, scols);
+    load_matrix(Ss, sv, sr, sr, true);
+  }
+
+  auto poison = [&]() {
+    __syncthreads();
+    if (tid == 0) {
+      if (c >= 0) ktrsv::st_release(&flags[tidx(i, c)], -1);
+      if (diag) ktrsv::st_release(&flags[tidx(i, i)], -1);
+    }
+  };
+  auto wait2 = [&](int k) {  // thread 0
+    const int a = ktrsv::wait_flag(&flags[tidx(i, k)], g.err);
+    return a < 0 ? -1 : ktrsv::wait_flag(&flags[tidx(c, k)], g.err);
+  };
+  auto fetch = [&](int k) {
+    fetch_tile(A0 + (k & 1) * TILE, g.ws + (int64_t)tidx(i, k) * TILE);
+    fetch_tile(B0 + (k & 1) * TILE, g.ws + (int64_t)tidx(c, k) * TILE);
+  };
+
+  if (c > 0) {
+    T acc[8][8];
+#pragma unroll
+    for (int p = 0; p < 8; ++p)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[p][q] = T(0);
+    if (tid == 0) sh_state = wait2(0);
+    __syncthreads();
+    if (sh_state < 0) return poison();
+    fetch(0);
+    ktrsv::cp_commit();
+    for (int k = 0; k < c; ++k) {
+      const bool more = k + 1 < c;
+      if (tid == 0)
+        sh_ready[k & 1] = more ? peek2(&flags[tidx(i, k + 1)], &flags[tidx(c, k + 1)]) : 0;
+      ktrsv::cp_wait_all();
+      __syncthreads();  // tile k landed; every thread is done with the other buffers
+      const bool ready = more && sh_ready[k & 1] > 0;
+      if (ready) fetch(k + 1);
+      ktrsv::cp_commit();
+      const T* Ak = A0 + (k & 1) * TILE;
+      const T* Bk = B0 + (k & 1) * TILE;
+      if (!diag) product8<NB / G>(acc, Ak, Bk, grp * (NB / G), u);
+      else
+        product8<2 * NB / G>(acc, Ak, grp < G / 2 ? Bk : Ak, (grp % (G / 2)) * (2 * NB / G), u);
+      if (more && !ready) {
+        if (tid == 0) sh_state = wait2(k + 1);
+        __syncthreads();
+        if (sh_state < 0) return poison();
+        fetch(k + 1);
+        ktrsv::cp_commit();
+      }
+    }
+    // T := A_ic - acc, S := A_ii - sum L_ik L_ik^T (both still ahead of W_c);
+    // the partial sums meet in the operand buffers (4 tiles)
+    __syncthreads();
+    if constexpr (G == 8) {
+      if (!diag) {
+        if (grp >= 4) store8(A0 + (grp - 4) * TILE, acc, u);
+        __syncthreads();
+        if (grp < 4) {
+          add8(acc, A0 + grp * TILE, u);
+          store8(A0 + grp * TILE, acc, u);
+        }
+        __syncthreads();
+        subtract<4>(Ts, A0);
+      } else {
+        if (grp < 4) store8(A0 + grp * TILE, acc, u);
+        __syncthreads();
+        subtract<4>(Ts, A0);
+        __syncthreads();
+        if (grp >= 4) store8(A0 + (grp - 4) * TILE, acc, u);
+        __syncthreads();
+        subtract<4>(Ss, A0);
+      }
+    } else {
+      store8(A0 + grp * TILE, acc, u);
+      __syncthreads();
+      if (!diag) {
+        subtract<4>(Ts, A0);
+      } else {
+        subtract<2>(Ts, A0);
+        subtract<2>(Ss, A0 + 2 * TILE);
+      }
+    }
+  }
+
+  T* Xs = A0;                // L_ic, k-major
+  T* Wc = A0 + TILE;         // W_c
+  T* red = B0;               // partial sums of the chain's products
+  T* Lb = B0 + TILE;         // L10, column-major, stride 32
+  T* Pb = Lb + 32 * 32;      // L10 inv(D0), column-major, stride 36
+  T* raw = Pb + 32 * 36;     // factor32's unscaled columns
+  T* out = g.ws + (c >= 0 ? (int64_t)tidx(i, c) * TILE : 0);
+  if (c >= 0) {
+    if (tid == 0) sh_state = ktrsv::wait_flag(&flags[tidx(c, c)], g.err);
+    __syncthreads();
+    if (sh_state < 0) return poison();
+    fetch_tile(Wc, g.ws + (int64_t)tidx(c, c) * TILE);
+    ktrsv::cp_commit();
+    ktrsv::cp_wait_all();
+    __syncthreads();
+    // X = T W_c^T, rows 0-31 (diagonal CTAs) or all rows: 4 x 4 per thread,
+    // groups of threads split k (W_c(c, k) = 0 for k > c)
+    T o[4][4];
+    if (!diag) {
+      constexpr int XG = THR / 256, KX = NB / XG;
+      const int xg = tid >> 8, v = tid & 255, tr = v & 15, tc = v >> 4;
+      product4<NB, NB>(o, Ts, Wc, xg * KX, min(xg * KX + KX, tc * 4 + 4), tr, tc);
+      reduce4<XG, 256, 1>(o, red, xg, v);
+      if (xg == 0) {
+        put4<NB, false>(Xs, o, tr, tc);
+        put4<NB, false>(out, o, tr, tc);
+      }
+      __syncthreads();
+      if (tid == 0) ktrsv::st_release(&flags[tidx(i, c)], 1);
+      store_matrix(Xs, xv, xr, xc, false);
+      return;
+    }
+    {
+      constexpr int XG = THR / 128, KX = NB / XG;
+      const int xg = tid >> 7, v = tid & 127, tr = v & 7, tc = v >> 3;
+      product4<NB, NB>(o, Ts, Wc, xg * KX, min(xg * KX + KX, tc * 4 + 4), tr, tc);
+      reduce4<XG, 128, 1>(o, red, xg, v);
+      if (xg == 0) {
+        put4<NB, false>(Xs, o, tr, tc);
+        put4<NB, false>(out, o, tr, tc);
+      }
+    }
+    __syncthreads();
+    // S00 -= X0 X0^T
+    {
+      constexpr int SG = THR / 64, KS = NB / SG;
+      const int tr = u & 7, tc = u >> 3;
+      product4<NB, NB>(o, Xs, Xs, grp * KS, grp * KS + KS, tr, tc);
+      reduce4<SG, 64, 1>(o, red, grp, u);
+      if (grp == 0) put4<NB, true>(Ss, o, tr, tc);
+    }
+  }
+  __syncthreads();
+
+  // Diagonal tile by 32 x 32 quarters: D0 and its inverse by warps 0 and 1,
+  // while the last quarter of the warps on the SMSPs that hold neither form
+  // X's lower rows and the rest of S.
+  constexpr int SH = THR / 2;  // threads of the shadow work: warps w with w % 4 >= 2
+  const bool shadow = (warp & 3) >= 2;
+  const int st = ((warp >> 2) * 2 + (warp & 1)) * 32 + lane;
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {  // one copy of the code (instruction cache)
+    if (warp == 0) {
+      const int f = factor32(Ss + h * (32 * NB + 32), raw, 2 + 4 * h);
+      if (lane == 0 && f) sh_fail = 32 * h + f;
+    } else if (warp == 1) {
+      inverse32(Ws + h * (32 * LDW + 32), raw, 2 + 4 * h);
+    } else if (h == 0 && shadow) {
+      if (c >= 0) {
+        T o[4][4];
+        {
+          constexpr int XG = SH / 128, KX = NB / XG;
+          const int xg = st >> 7, v = st & 127, tr = v & 7, tc = v >> 3;
+          product4<NB, NB>(o, Ts + 32, Wc, xg * KX, min(xg * KX + KX, tc * 4 + 4), tr, tc);
+          reduce4<XG, 128, 10>(o, red, xg, v);
+          if (xg == 0) {
+            put4<NB, false>(Xs + 32, o, tr, tc);
+            put4<NB, false>(out + 32, o, tr, tc);
+          }
+        }
+        bar_sync<10, SH>();
+        {
+          // S10 -= X1 X0^T and S11 -= X1 X1^T, 64 threads each
+          constexpr int SG = SH / 128, KS = NB / SG;
+          const int sg = st >> 7, v = st & 127, w = v & 63, q11 = v >> 6, tr = w & 7, tc = w >> 3;
+          product4<NB, NB>(o, Xs + 32, Xs + 32 * q11, sg * KS, sg * KS + KS, tr, tc);
+          reduce4<SG, 128, 10>(o, red, sg, v);
+          if (sg == 0) put4<NB, true>(Ss + 32 * q11 * NB + 32, o, tr, tc);
+        }
+        if (st == SH - 1) ktrsv::st_release(&flags[tidx(i, c)], 1);  // X, ordered by the barriers
+      }
+      for (int e = st; e < 32 * 32; e += SH) Ws[(32 + (e >> 5)) * LDW + (e & 31)] = T(0);
+    } else if (h == 1 && shadow) {
+      // off the chain: L10 into S's lower-left quarter, P = L10 inv(D0)
+      for (int cc = st >> 5; cc < 32; cc += SH / 32) {
+        Ss[cc * NB + 32 + lane] = Lb[cc * 32 + lane];
+        T o = T(0);
+#pragma unroll 4
+        for (int k = 0; k < 32; k += 4) {
+          T b[4];
+          lds4(Ws + cc * LDW + k, b);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) o = fma(Lb[(k + q) * 32 + lane], b[q], o);
+        }
+        Pb[cc * 36 + lane] = o;
+      }
+    }
+    __syncthreads();
+    if (sh_fail || h == 1) break;
+    // L10 = S10 inv(D0)^T, then S11 -= L10 L10^T: 4 x 4 on two groups of 64
+    T o[4][4];
+    const int tr = u & 7, tc = u >> 3;
+    if (grp < 2) {
+      product4<NB, LDW>(o, Ss + 32, Ws, grp * 16, min(grp * 16 + 16, tc * 4 + 4), tr, tc);
+      reduce4<2, 64, 1>(o, red, grp, u);
+      if (grp == 0) put4<32, false>(Lb, o, tr, tc);
+      bar_sync<1, 128>();
+      product4<32, 32>(o, Lb, Lb, grp * 16, grp * 16 + 16, tr, tc);
+      reduce4<2, 64, 1>(o, red + 1024, grp, u);
+      if (grp == 0) put4<NB, true>(Ss + 32 * NB + 32, o, tr, tc);
+    }
+    __syncthreads();
+  }
+  if (!sh_fail) {
+    // W10 = -inv(D1) P
+    for (int c0 = warp * 2; c0 < 32; c0 += NW * 2) {
+      T o[2] = {T(0), T(0)};
+#pragma unroll
+      for (int k = 0; k < 32; k += 4) {
+        T p0[4], p1[4];
+        lds4(Pb + c0 * 36 + k, p0);
+        lds4(Pb + (c0 + 1) * 36 + k, p1);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const T a = Ws[(32 + k + q) * LDW + 32 + lane];
+          o[0] = fma(-a, p0[q], o[0]);
+          o[1] = fma(-a, p1[q], o[1]);
+        }
+      }
+      Ws[c0 * LDW + 32 + lane] = o[0];
+      Ws[(c0 + 1) * LDW + 32 + lane] = o[1];
+    }
+    __syncthreads();
+    T* wout = g.ws + (int64_t)tidx(i, i) * TILE;
+#pragma unroll
+    for (int w = 0; w < TILE / 4 / THR; ++w) {
+      const int e = tid + THR * w;
+      T v[4];
+      lds4(Ws + (e >> 4) * LDW + (e & 15) * 4, v);
+      sts4(wout + e * 4, v);
+    }
+    __syncthreads();
+    if (tid == 0) ktrsv::st_release(&flags[tidx(i, i)], 1);
+  } else if (tid == 0) {
+    const int col0 = i >= g.nb1 ? g.n1 + (i - g.nb1) * NB : i * NB;
+    atomicMin(g.info, g.info_base + col0 + sh_fail);
+    ktrsv::st_release(&flags[tidx(i, i)], -1);
+  }
+  if (c >= 0) store_matrix(Xs, xv, xr, xc, false);
+  store_matrix(Ss, sv, sr, sr, true);
+}
+
+}  // namespace kchol
+}  // namespace rfp

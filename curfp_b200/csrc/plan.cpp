@@ -137,12 +137,16 @@ int potrf_lower(ExecT<T>& ex, ViewT<T> A, int n, int info_base, int math) {
   if (n <= 0) return 0;
   const int tile = ex.potrf_tile_rows();
   if (n <= tile) return ex.potrf_tile(A, n, info_base);
-  int n1 = split(n, tile), n2 = n - n1;
-  int rc = potrf_lower(ex, A, n1, info_base, math);
-  if (rc) return rc;
+  int n1 = split(n, kPotrfTile), n2 = n - n1;
   ViewT<T> A21 = sub(A, n1, 0);
-  // A21 := A21 L11^{-T}   <=>   L11 A21^T = A21^T
-  if ((rc = trsm_lln(ex, A, n1, tr(A21), n2, 1.0f, math))) return rc;
+  int rc;
+  if (ex.has_panel(n1, n2)) {
+    if ((rc = ex.potrf_panel(A, A21, n1, n2, info_base))) return rc;
+  } else {
+    if ((rc = potrf_lower(ex, A, n1, info_base, math))) return rc;
+    // A21 := A21 L11^{-T}   <=>   L11 A21^T = A21^T
+    if ((rc = trsm_lln(ex, A, n1, tr(A21), n2, 1.0f, math))) return rc;
+  }
   // A22 := A22 - A21 A21^T (lower)
   SharedTaskT<T> t{0, 0, n2, n2, sub(A, n1, n1), -1.0f, 1.0f, 1};
   if ((rc = ex.gemm_shared(A21, n2, n1, &t, 1, math))) return rc;
@@ -232,12 +236,16 @@ int spftrf(ExecT<T>& ex, int transr, int lower, int n, T* A, int math) {
   Geometry g = geometry(n, transr, lower);
   ViewT<T> V11 = block_view(A, g.b11), V21 = block_view(A, g.b21),
        V22 = block_view(A, g.b22);
-  int rc = potrf_lower(ex, V11, g.n1, 0, math);
-  if (rc) return rc;
+  int rc = ex.potrf_blocks(V11, V21, V22, g.n1, g.n2);
+  if (rc != kNotSupported) return rc;
+  const bool panel = ex.has_panel(g.n1, g.n2);
+  if (!panel && (rc = potrf_lower(ex, V11, g.n1, 0, math))) return rc;
   if ((rc = ex.after_first_block())) return rc;
   if (g.n2 == 0) return 0;
   if (g.n1 > 0) {
-    if ((rc = trsm_lln(ex, V11, g.n1, tr(V21), g.n2, 1.0f, math))) return rc;
+    rc = panel ? ex.potrf_panel(V11, V21, g.n1, g.n2, 0)
+               : trsm_lln(ex, V11, g.n1, tr(V21), g.n2, 1.0f, math);
+    if (rc) return rc;
     SharedTaskT<T> t{0, 0, g.n2, g.n2, V22, -1.0f, 1.0f, 1};
     if ((rc = ex.gemm_shared(V21, g.n2, g.n1, &t, 1, math))) return rc;
   }
