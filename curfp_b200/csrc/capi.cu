@@ -181,6 +181,7 @@ curfpStatus_t curfpDestroy(curfpHandle_t handle) {
   if (handle->ws3) cudaFree(handle->ws3);
   if (handle->tsv) cudaFree(handle->tsv);
   if (handle->wsg) cudaFree(handle->wsg);
+  if (handle->wst) cudaFree(handle->wst);
   if (handle->d_info) cudaFree(handle->d_info);
   if (handle->copy_stream) {
     cudaStreamSynchronize(handle->copy_stream);
@@ -203,12 +204,12 @@ curfpStatus_t curfpReleaseWorkspace(curfpHandle_t handle) {
     return CURFP_STATUS_EXECUTION_FAILED;
   }
   void** bufs[] = {&handle->ws, &handle->stage, &handle->stage2, &handle->ws2,
-                   &handle->ws3, &handle->tsv, &handle->wsg};
+                   &handle->ws3, &handle->tsv, &handle->wsg, &handle->wst};
   size_t* sizes[] = {&handle->ws_bytes, &handle->stage_bytes, &handle->stage2_bytes,
                      &handle->ws2_bytes, &handle->ws3_bytes, &handle->tsv_bytes,
-                     &handle->wsg_bytes};
+                     &handle->wsg_bytes, &handle->wst_bytes};
   bool ok = true;
-  for (int i = 0; i < 7; ++i) {
+  for (int i = 0; i < 8; ++i) {
     if (*bufs[i]) ok &= cudaFree(*bufs[i]) == cudaSuccess;
     *bufs[i] = nullptr;
     *sizes[i] = 0;

@@ -37,6 +37,8 @@ struct curfpContext {
   rfp::Profiler prof;      // optional per-class event timing
   void* tsv = nullptr;     // wavefront solve flags / tickets
   size_t tsv_bytes = 0;
+  void* wst = nullptr;     // tiles published by the wavefront solves, packed operand copies
+  size_t wst_bytes = 0;
   void* wsg = nullptr;     // adjoint scratch (solve adjoint n x 2nrhs, NLL gradient)
   size_t wsg_bytes = 0;
   cudaStream_t copy_stream = nullptr;  // host-input factorization: the overlapped copy
@@ -52,6 +54,16 @@ namespace rfp {
 constexpr int kCholRows = 2048;
 constexpr int kCholPanelRows = 2048;
 constexpr int kCholRfpRows = 4096;
+// Triangular inverses of up to kTriRows are one wave; L^T L products and
+// in-place triangular multiplies of up to kLeafRows are one masked product on
+// the SIMT cores (on a copy of the operand).  Not on the tensor cores: a row's
+// digits are relative to its largest element, and an inverse factor's rows
+// have a dominant diagonal (n = 6001 inverse, error against FP64: 1.8e-5 with
+// 2048-row blocks on the tensor cores, 5e-7 with the diagonal kept apart,
+// 1.9e-7 this way).  1024 against 512 rows: 6.2 against 7.5 ms for that
+// inverse (25.6 ms with 64-row leaves).
+constexpr int kTriRows = 2048;
+constexpr int kLeafRows = 1024;
 
 // The CUDA executor for FP32 (SIMT and split-BF16 tensor-core contractions)
 // and FP64 (SIMT DFMA) element types.
@@ -70,7 +82,11 @@ class CudaExecT : public ExecT<T> {
   int trtri_tile(ViewT<T> L, int n) override;
   int lauum_tile(ViewT<T> L, int n) override;
   T* workspace(size_t count) override;
-  int inplace_rows() const override { return 64; }
+  int trtri_rows() const override { return kTriRows; }
+  int trtri_block(ViewT<T> L, int n) override;
+  int lauum_rows() const override { return kLeafRows; }
+  int lauum_block(ViewT<T> L, int n) override;
+  int inplace_rows() const override { return kLeafRows; }
   int gemm_shared(ViewT<T> X, int rows, int k, const SharedTaskT<T>* t, int count,
                   int math) override;
   int gemm_pair(ViewT<T> X, ViewT<T> Y, int rows, int k, const SharedTaskT<T>* t, int count,

@@ -69,12 +69,8 @@ constexpr int kTrsmLeaf = 64;    // TRSM diagonal blocks (inverted, then multipl
 constexpr int kInvStride = 2 * kTrsmLeaf * kTrsmLeaf;
 constexpr int kTriTile = 64;     // trtri / lauum tiles
 constexpr int kAdjTile = 64;     // Cholesky-adjoint diagonal tiles
-constexpr int kTrmmLeaf = 64;    // TRMM leaves (masked in-place multiply)
 constexpr int kTrsvMaxRhs = 512; // wavefront solve for at most this many RHS
-constexpr int kTrsvMaxRhsTc = 64;  // ... when the updates may use the tensor cores
 constexpr int kWaveLeaf = 512;   // recursive TRSM hands blocks <= this to the wavefront solve
-constexpr int kWaveLeafWide = 512;  // ... when there are more than 4 * kTrsvMaxRhs RHS
-constexpr int kWaveLeafWideTc = 512;  // ... and the updates may use the tensor cores
 constexpr int kNotSupported = -1;
 
 template <typename T>
@@ -119,6 +115,12 @@ class ExecT {
   virtual int trtri_tile(ViewT<T> L, int n) = 0;
   // In-place L := L^T L (lower triangle; n <= kTriTile).
   virtual int lauum_tile(ViewT<T> L, int n) = 0;
+  // The same two operations on larger blocks, of up to trtri_rows() and
+  // lauum_rows(), which the recursions end in.
+  virtual int trtri_rows() const { return kTriTile; }
+  virtual int trtri_block(ViewT<T> L, int n) { return trtri_tile(L, n); }
+  virtual int lauum_rows() const { return kTriTile; }
+  virtual int lauum_block(ViewT<T> L, int n) { return lauum_tile(L, n); }
   // Scratch of at least count elements, valid until the next workspace() call.
   virtual T* workspace(size_t count) = 0;
   // Largest m of an in-place GEMM.

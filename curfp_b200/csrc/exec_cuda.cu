@@ -10,6 +10,7 @@
 #include "gemm_route.h"
 #include "k_skinny.cuh"
 #include "k_tile.cuh"
+#include "k_tri.cuh"
 #include "k_trsv.cuh"
 
 namespace rfp {
@@ -117,6 +118,70 @@ int launch_skinny(const GemmProbT<T>& g0, const int* abort_flag, curfpContext* c
 
 }  // namespace
 
+namespace {
+// Dst (packed, Src's contiguous dimension first) := Src (rows x cols view);
+// lower: only elements with row >= column.  The warp runs along the
+// contiguous dimension.
+template <typename T>
+__global__ void __launch_bounds__(256) copy_view(ViewT<T> dst, ViewT<T> src, int rows, int cols,
+                                                 int lower, const int* abort_flag) {
+  if (abort_flag && *abort_flag != INT_MAX) return;
+  const bool rowcont = (src.cs == 1 || src.cs == -1) && !(src.rs == 1 || src.rs == -1);
+  const int64_t inner = rowcont ? cols : rows, total = (int64_t)rows * cols;
+  for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < total;
+       e += (int64_t)gridDim.x * 256) {
+    const int64_t o = e / inner, k = e % inner;
+    const int64_t r = rowcont ? o : k, c = rowcont ? k : o;
+    if (!lower || r >= c) dst.p[r * dst.rs + c * dst.cs] = src.p[r * src.rs + c * src.cs];
+  }
+}
+
+// L(i, j) := s(i, i) s(i, j) on the lower triangle.
+template <typename T>
+__global__ void __launch_bounds__(256) scale_by_diagonal(ViewT<T> L, ViewT<T> s, int n,
+                                                         const int* abort_flag) {
+  if (abort_flag && *abort_flag != INT_MAX) return;
+  const bool rowcont = (L.cs == 1 || L.cs == -1) && !(L.rs == 1 || L.rs == -1);
+  const int64_t total = (int64_t)n * n;
+  for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < total;
+       e += (int64_t)gridDim.x * 256) {
+    const int64_t o = e / n, k = e % n;
+    const int64_t i = rowcont ? o : k, j = rowcont ? k : o;
+    if (i >= j) L.p[i * L.rs + j * L.cs] = s.p[i * (s.rs + s.cs)] * s.p[i * s.rs + j * s.cs];
+  }
+}
+
+// A packed copy of a view in the handle's tile workspace.
+template <typename T>
+int packed_copy(curfpContext* ctx, const int* abort_flag, ViewT<T> src, int rows, int cols,
+                int lower, ViewT<T>* out) {
+  const int64_t total = (int64_t)rows * cols;
+  T* p = static_cast<T*>(
+      grow_buffer(ctx, &ctx->wst, &ctx->wst_bytes, (size_t)total * sizeof(T)));
+  if (!p) return 2;
+  const bool rowcont = (src.cs == 1 || src.cs == -1) && !(src.rs == 1 || src.rs == -1);
+  *out = rowcont ? ViewT<T>{p, cols, 1} : ViewT<T>{p, 1, rows};
+  const int64_t blocks = (total + 1023) / 1024;
+  ProfScope ps(ctx->prof, ctx->stream, K_PACK, 0, 2.0 * sizeof(T) * total);
+  copy_view<T><<<(int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, ctx->stream>>>(
+      *out, src, rows, cols, lower, abort_flag);
+  ++ctx->launches;
+  return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+
+// An in-place SIMT problem of more than one tile row reads a copy of B.
+template <typename T>
+int unalias(curfpContext* ctx, const int* abort_flag, GemmProbT<T>* g) {
+  if (!g->inplace || g->m <= 64) return 0;
+  ViewT<T> b;
+  const int rc = packed_copy(ctx, abort_flag, g->B, g->k, g->n, 0, &b);
+  if (rc) return rc;
+  g->B = g->B2 = b;
+  g->inplace = 0;
+  return 0;
+}
+}  // namespace
+
 // Output written through a column-contiguous view keeps the tensor-core
 // epilogue's warp-wide stores coalesced: C = A B^T is computed as
 // C^T = B A^T when C's contiguous dimension is its column index.
@@ -198,6 +263,13 @@ int CudaExecT<double>::gemm(const GemmProbT<double>* p, int count) {
     const int rc = launch_skinny<double>(p[0], abort_, ctx_);
     if (rc >= 0) return rc;
   }
+  GemmProbT<double> q;
+  if (count == 1 && p[0].inplace) {
+    q = p[0];
+    const int rc = unalias(ctx_, abort_, &q);
+    if (rc) return rc;
+    p = &q;
+  }
   // 128 x 128 tiles (64 accumulators per thread, one CTA per SM) when they
   // fill the machine, else 64 x 64
   int64_t t128 = 0;
@@ -246,6 +318,13 @@ int CudaExecT<float>::gemm(const GemmProb* p, int count) {
       if (rc) return rc;
     }
     return 0;
+  }
+  GemmProb q;
+  if (count == 1 && p[0].inplace) {
+    q = p[0];
+    const int rc = unalias(ctx_, abort_, &q);
+    if (rc) return rc;
+    p = &q;
   }
   // Tile choice: 128 x 128 when it fills the machine, else 64 x 64.
   int64_t t128 = 0;
@@ -373,6 +452,40 @@ int CudaExecT<T>::trtri_tile(ViewT<T> L, int n) {
 }
 
 template <typename T>
+int CudaExecT<T>::trtri_block(ViewT<T> L, int n) {
+  if (n <= 0) return 0;
+  if (n <= ktile::T) return trtri_tile(L, n);
+  const int nblk = (n + kTrsmLeaf - 1) / kTrsmLeaf;
+  T* W = workspace((size_t)nblk * kInvStride);
+  if (!W) return 2;
+  const int rc = trtri_blocks(L, n, kTrsmLeaf, W);
+  if (rc) return rc;
+  ktri::Args<T> a{};
+  a.L = L;
+  a.n = n;
+  a.W = W;
+  const int tiles = nblk * (nblk + 1) / 2;
+  const size_t words = 1 + (size_t)tiles;
+  a.ws = static_cast<T*>(grow_buffer(ctx_, &ctx_->wst, &ctx_->wst_bytes,
+                                     (size_t)tiles * ktri::TILE * sizeof(T)));
+  a.sync = static_cast<int*>(grow_buffer(ctx_, &ctx_->tsv, &ctx_->tsv_bytes, words * sizeof(int)));
+  if (!a.ws || !a.sync) return 2;
+  if (cudaMemsetAsync(a.sync, 0, words * sizeof(int), ctx_->stream) != cudaSuccess) return 4;
+  a.err = ctx_->d_info + 1;
+  a.abort_flag = abort_;
+  constexpr int smem = ktri::smem_bytes<T>();
+  static const bool attr = smem_attr(ktri::inverse_wave<T>, smem);
+  if (!attr) return 4;
+  ProfScope ps(ctx_->prof, ctx_->stream, K_TRTRI, (double)n * n * n / 3, 0);
+  ps.shape(n, n, n, tiles);
+  ktri::inverse_wave<T><<<tiles, ktri::THR, smem, ctx_->stream>>>(a);
+  ktri::store_inverse<T><<<tiles, ktri::THR, 0, ctx_->stream>>>(L, n, a.ws, abort_);
+  ctx_->launches += 2;
+  ++ctx_->wait_launches;
+  return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+
+template <typename T>
 int CudaExecT<T>::lauum_tile(ViewT<T> L, int n) {
   if (n <= 0) return 0;
   if (n > ktile::T) return 3;
@@ -380,6 +493,35 @@ int CudaExecT<T>::lauum_tile(ViewT<T> L, int n) {
   ktile::lauum_tile<T><<<1, 256, 0, ctx_->stream>>>(L, n);
   ++ctx_->launches;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+
+// L := L^T L (lower) as one product: with L = D + N,
+// (L^T L)(i, j) = d_i L(i, j) + (N^T N)(i, j) for i >= j, masked operands read
+// from a packed copy of L.  (A sum that starts at a dominant d_i^2 rounds every
+// later term against it: diagonal error 2.4e-6 against 7e-7 at n = 6001.)
+template <typename T>
+int CudaExecT<T>::lauum_block(ViewT<T> L, int n) {
+  if (n <= ktile::T) return lauum_tile(L, n);
+  ViewT<T> c;
+  const int rc = packed_copy(ctx_, abort_, L, n, n, 1, &c);
+  if (rc) return rc;
+  GemmProbT<T> p{};
+  p.A = p.A2 = tr(c);
+  p.B = p.B2 = c;
+  p.C = L;
+  p.m = p.n = p.k = n;
+  p.alpha = p.beta = T(1);
+  p.c_lower = 1;
+  p.a_tri = 3;
+  p.b_tri = 1;
+  {
+    ProfScope ps(ctx_->prof, ctx_->stream, K_LAUUM, 0, 0);
+    const int64_t blocks = ((int64_t)n * n + 1023) / 1024;
+    scale_by_diagonal<T><<<(int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, ctx_->stream>>>(
+        L, c, n, abort_);
+    ++ctx_->launches;
+  }
+  return gemm(&p, 1);
 }
 
 namespace {

@@ -15,11 +15,9 @@
 // and, when i = c + 1, it also factors the next diagonal tile,
 //   S    = A_ii - sum_{k<c} L_ik L_ik^T - X X^T = L_ii L_ii^T,  W_i = inv(L_ii).
 //
-// The sums run on 8 x 8 register tiles: shared memory returns 128 bytes a
-// cycle, so a 4 x 4 tile (8 loads for 16 FMAs) would run at half the FMA rate
-// and 8 x 8 is where the two meet.  64 threads cover a tile; the CTA's groups
-// of 64 threads split k and their partial sums meet once per CTA.  In a
-// diagonal CTA half of the groups sum for X and half for S.
+// The sums run on 8 x 8 register tiles (k_micro.cuh): 64 threads cover a tile,
+// the CTA's groups of 64 split k and their partial sums meet once per CTA.  In
+// a diagonal CTA half of the groups sum for X and half for S.
 //
 // The chain from one W to the next is ordered so that only what the next
 // pivot needs is on it: X's upper 32 rows, S's upper-left quarter, its factor
@@ -49,14 +47,14 @@
 #include <cstdint>
 
 #include "engine.h"
-#include "k_tile.cuh"
+#include "k_micro.cuh"
 #include "k_trsv.cuh"
 
 namespace rfp {
 namespace kchol {
 
-constexpr int NB = 64;
-constexpr int TILE = NB * NB;
+using namespace kmicro;
+
 constexpr int LDW = NB + 4;  // column stride of W in shared memory (conflict-free 16-byte columns)
 
 // 64 threads per group; FP32 has 512 threads, FP64 256 (registers).
@@ -93,11 +91,6 @@ inline int cta_count(int nb, int nbf) {
   return t;
 }
 
-// 16 bytes by cp.async, L2 only (the data was written by CTAs of this launch).
-__device__ __forceinline__ void cp16(void* smem, const void* g) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(g) : "memory");
-}
 template <typename T>
 __device__ __forceinline__ void fetch_tile(T* s, const T* g) {
   constexpr int VW = 16 / (int)sizeof(T);
@@ -107,10 +100,6 @@ __device__ __forceinline__ void fetch_tile(T* s, const T* g) {
     cp16(s + e, g + e);
   }
 }
-template <int ID, int COUNT>
-__device__ __forceinline__ void bar_sync() {
-  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(COUNT) : "memory");
-}
 template <int COUNT>
 __device__ __forceinline__ void bar_sync_id(int id) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(COUNT) : "memory");
@@ -118,137 +107,6 @@ __device__ __forceinline__ void bar_sync_id(int id) {
 template <int COUNT>
 __device__ __forceinline__ void bar_arrive_id(int id) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(COUNT) : "memory");
-}
-
-using ktrsv::lds4;
-__device__ __forceinline__ void sts4(float* p, const float (&v)[4]) {
-  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-__device__ __forceinline__ void sts4(double* p, const double (&v)[4]) {
-  reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
-  reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
-}
-
-// acc += A B^T over k in [k0, k0 + KG), A and B k-major (column stride 64);
-// thread u of 64: rows 4 (u % 8) + {0, 32}.., columns 4 (u / 8) + {0, 32}..
-template <int KG, typename T>
-__device__ __forceinline__ void product8(T (&acc)[8][8], const T* A, const T* B, int k0, int u) {
-  const T* a0 = A + k0 * NB + (u & 7) * 4;
-  const T* b0 = B + k0 * NB + (u >> 3) * 4;
-#pragma unroll 4
-  for (int k = 0; k < KG; ++k) {
-    T a[8], b[8];
-    lds4(a0 + k * NB, *reinterpret_cast<T(*)[4]>(a));
-    lds4(a0 + k * NB + 32, *reinterpret_cast<T(*)[4]>(a + 4));
-    lds4(b0 + k * NB, *reinterpret_cast<T(*)[4]>(b));
-    lds4(b0 + k * NB + 32, *reinterpret_cast<T(*)[4]>(b + 4));
-#pragma unroll
-    for (int p = 0; p < 8; ++p)
-#pragma unroll
-      for (int q = 0; q < 8; ++q) acc[p][q] = fma(a[p], b[q], acc[p][q]);
-  }
-}
-template <typename T>
-__device__ __forceinline__ void store8(T* s, const T (&acc)[8][8], int u) {
-#pragma unroll
-  for (int q = 0; q < 8; ++q)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const T v[4] = {acc[4 * h][q], acc[4 * h + 1][q], acc[4 * h + 2][q], acc[4 * h + 3][q]};
-      sts4(s + ((u >> 3) * 4 + (q >> 2) * 32 + (q & 3)) * NB + (u & 7) * 4 + 32 * h, v);
-    }
-}
-template <typename T>
-__device__ __forceinline__ void add8(T (&acc)[8][8], const T* s, int u) {
-#pragma unroll
-  for (int q = 0; q < 8; ++q)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      T v[4];
-      lds4(s + ((u >> 3) * 4 + (q >> 2) * 32 + (q & 3)) * NB + (u & 7) * 4 + 32 * h, v);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[4 * h + e][q] += v[e];
-    }
-}
-// dst -= the sum of N partial tiles at src, src + TILE, ... (all threads).
-template <int N, typename T>
-__device__ __forceinline__ void subtract(T* dst, const T* src) {
-#pragma unroll
-  for (int w = 0; w < TILE / 4 / threads<T>(); ++w) {
-    const int e = (threadIdx.x + threads<T>() * w) * 4;
-    T s[4], v[4];
-    lds4(src + e, s);
-#pragma unroll
-    for (int i = 1; i < N; ++i) {
-      lds4(src + i * TILE + e, v);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) s[q] += v[q];
-    }
-    lds4(dst + e, v);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] -= s[q];
-    sts4(dst + e, v);
-  }
-}
-
-// out(4 x 4 at rows 4 tr, columns 4 tc) = sum_{k0 <= k < k1} A B^T, column
-// strides LDA, LDB.
-template <int LDA, int LDB, typename T>
-__device__ __forceinline__ void product4(T (&o)[4][4], const T* A, const T* B, int k0, int k1,
-                                         int tr, int tc) {
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) o[p][q] = T(0);
-#pragma unroll 4
-  for (int k = k0; k < k1; ++k) {
-    T a[4], b[4];
-    lds4(A + k * LDA + tr * 4, a);
-    lds4(B + k * LDB + tc * 4, b);
-#pragma unroll
-    for (int p = 0; p < 4; ++p)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) o[p][q] = fma(a[p], b[q], o[p][q]);
-  }
-}
-// The sum over G groups of CNT threads each (thread u of group g; COUNT =
-// G * CNT threads meet at barrier ID) into group 0; red: (G - 1) * CNT * 16.
-template <int G, int CNT, int ID, typename T>
-__device__ __forceinline__ void reduce4(T (&o)[4][4], T* red, int g, int u) {
-  if constexpr (G > 1) {
-    if (g > 0) {
-#pragma unroll
-      for (int p = 0; p < 4; ++p) sts4(red + (((g - 1) * 4 + p) * CNT + u) * 4, o[p]);
-    }
-    bar_sync<ID, G * CNT>();
-    if (g == 0) {
-#pragma unroll
-      for (int i = 0; i < G - 1; ++i)
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          T v[4];
-          lds4(red + ((i * 4 + p) * CNT + u) * 4, v);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) o[p][q] += v[q];
-        }
-    }
-  }
-}
-// s(rows 4 tr.., columns 4 tc..; column stride LD) = o, or -= o.
-template <int LD, bool kSub, typename T>
-__device__ __forceinline__ void put4(T* s, const T (&o)[4][4], int tr, int tc) {
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    T* p = s + (tc * 4 + q) * LD + tr * 4;
-    T v[4] = {o[0][q], o[1][q], o[2][q], o[3][q]};
-    if (kSub) {
-      T w[4];
-      lds4(p, w);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = w[e] - v[e];
-    }
-    sts4(p, v);
-  }
 }
 
 // 1/sqrt(d): the hardware estimate r and one Newton step for y = x^-1/2 in
@@ -349,32 +207,54 @@ __device__ __forceinline__ ViewT<T> tile_view(const Args<T>& g, int i, int j, in
   return sub(c2 ? g.v22 : (r2 ? g.v21 : g.v11), li, lj);
 }
 
+// Visits the tile's elements in groups of four rows of a column: group (b, q)
+// holds rows 4q .. 4q + 3 of column b, one 16-byte shared-memory access.  For
+// row-contiguous views a warp takes 8 columns x 4 groups (whole 32-byte
+// sectors in memory, 8 banks apart in shared memory, where lanes along a row
+// would all fall in one bank), else 16 groups x 2 columns.
+template <typename T, typename F>
+__device__ __forceinline__ void for_groups(bool rowcont, F f) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int NW = threads<T>() / 32;
+#pragma unroll
+  for (int u = 0; u < 32 / NW; ++u) {
+    const int w = warp + NW * u;
+    if (rowcont) f((w & 7) * 8 + (lane & 7), (w >> 3) * 4 + (lane >> 3));
+    else f(w * 2 + (lane >> 4), lane & 15);
+  }
+}
+
 // Matrix tile -> k-major shared tile, zeros (diag: identity) outside; of a
 // diagonal tile only the lower triangle is read and zeros stand above it.
 template <typename T>
 __device__ __forceinline__ void load_matrix(T* s, ViewT<T> v, int rows, int cols, bool diag) {
   const bool rowcont = (v.cs == 1 || v.cs == -1) && !(v.rs == 1 || v.rs == -1);
-#pragma unroll 4
-  for (int u = 0; u < TILE / threads<T>(); ++u) {
-    const int e = threadIdx.x + threads<T>() * u;
-    const int a = rowcont ? e / NB : e % NB, b = rowcont ? e % NB : e / NB;
-    T x = diag && a == b ? T(1) : T(0);
-    if (a < rows && b < cols && (!diag || a >= b))
-      x = __ldcg(v.p + (int64_t)a * v.rs + (int64_t)b * v.cs);
-    s[b * NB + a] = x;
-  }
+  for_groups<T>(rowcont, [&](int b, int q) {
+    T x[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int a = 4 * q + e;
+      x[e] = diag && a == b ? T(1) : T(0);
+      if (a < rows && b < cols && (!diag || a >= b))
+        x[e] = __ldcg(v.p + (int64_t)a * v.rs + (int64_t)b * v.cs);
+    }
+    sts4(s + b * NB + 4 * q, x);
+  });
 }
 template <typename T>
 __device__ __forceinline__ void store_matrix(const T* s, ViewT<T> v, int rows, int cols,
                                              bool diag) {
   const bool rowcont = (v.cs == 1 || v.cs == -1) && !(v.rs == 1 || v.rs == -1);
-#pragma unroll 4
-  for (int u = 0; u < TILE / threads<T>(); ++u) {
-    const int e = threadIdx.x + threads<T>() * u;
-    const int a = rowcont ? e / NB : e % NB, b = rowcont ? e % NB : e / NB;
-    if (a < rows && b < cols && (!diag || a >= b))
-      v.p[(int64_t)a * v.rs + (int64_t)b * v.cs] = s[b * NB + a];
-  }
+  for_groups<T>(rowcont, [&](int b, int q) {
+    T x[4];
+    lds4(s + b * NB + 4 * q, x);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int a = 4 * q + e;
+      if (a < rows && b < cols && (!diag || a >= b))
+        v.p[(int64_t)a * v.rs + (int64_t)b * v.cs] = x[e];
+    }
+  });
 }
 
 // Both flags ready: 1; either poisoned: -1; else 0.
@@ -385,14 +265,13 @@ __device__ __forceinline__ int peek2(const int* f, const int* g) {
 
 template <typename T>
 __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
-  if (g.info && *g.info != INT_MAX) return;
   extern __shared__ __align__(16) unsigned char chol_raw[];
   T* A0 = reinterpret_cast<T*>(chol_raw);  // L_ik, double-buffered
   T* B0 = A0 + 2 * TILE;                   // L_ck, double-buffered
   T* Ts = B0 + 2 * TILE;
   T* Ss = Ts + TILE;
   T* Ws = Ss + TILE;  // W_i, column stride LDW
-  __shared__ int sh_ticket, sh_ready[2], sh_state, sh_fail;
+  __shared__ int sh_ticket, sh_known[3], sh_state, sh_fail;
   constexpr int THR = threads<T>(), G = groups<T>();
   const int tid = threadIdx.x, grp = tid >> 6, u = tid & 63;
   const int warp = tid >> 5, lane = tid & 31;
@@ -401,6 +280,7 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
     sh_ticket = atomicAdd(g.sync, 1);
     sh_fail = 0;
   }
+  const bool abort = g.info && *g.info != INT_MAX;
   __syncthreads();
   int* flags = g.sync + 1;
   auto tidx = [&](int r, int k) { return tile_index(g.nbf, r, k); };
@@ -414,6 +294,15 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
   }
   const bool diag = i == c + 1 && i < g.nbf;
 
+  auto poison = [&]() {
+    __syncthreads();
+    if (tid == 0) {
+      if (c >= 0) ktrsv::st_release(&flags[tidx(i, c)], -1);
+      if (diag) ktrsv::st_release(&flags[tidx(i, i)], -1);
+    }
+  };
+  if (__syncthreads_or(abort)) return poison();  // a pivot failed earlier
+
   int xr = 0, xc = 0, sr = 0, scols = 0;
   ViewT<T> xv{}, sv{};
   if (c >= 0) {
@@ -425,16 +314,23 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
     load_matrix(Ss, sv, sr, sr, true);
   }
 
-  auto poison = [&]() {
-    __syncthreads();
-    if (tid == 0) {
-      if (c >= 0) ktrsv::st_release(&flags[tidx(i, c)], -1);
-      if (diag) ktrsv::st_release(&flags[tidx(i, i)], -1);
-    }
+  auto ready = [&](int k) { return peek2(&flags[tidx(i, k)], &flags[tidx(c, k)]); };
+  // Warp 0: how far from k on the tiles are published (32 flags in one round
+  // trip), into *known.
+  auto scan = [&](int k, int* known) {
+    const int st = k + lane < c ? ready(k + lane) : 0;
+    const unsigned m = __ballot_sync(0xffffffffu, st > 0);
+    if (lane == 0) *known = k + (m == 0xffffffffu ? 32 : __ffs(~m) - 1);
   };
-  auto wait2 = [&](int k) {  // thread 0
-    const int a = ktrsv::wait_flag(&flags[tidx(i, k)], g.err);
-    return a < 0 ? -1 : ktrsv::wait_flag(&flags[tidx(c, k)], g.err);
+  // Warp 0: waits for tile k, then scans on.
+  auto wait2 = [&](int k, int* known) {
+    if (lane == 0) {
+      int st = ktrsv::wait_flag(&flags[tidx(i, k)], g.err);
+      if (st > 0) st = ktrsv::wait_flag(&flags[tidx(c, k)], g.err);
+      sh_state = st;
+    }
+    __syncwarp();
+    scan(k, known);
   };
   auto fetch = [&](int k) {
     fetch_tile(A0 + (k & 1) * TILE, g.ws + (int64_t)tidx(i, k) * TILE);
@@ -447,29 +343,31 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
     for (int p = 0; p < 8; ++p)
 #pragma unroll
       for (int q = 0; q < 8; ++q) acc[p][q] = T(0);
-    if (tid == 0) sh_state = wait2(0);
+    if (warp == 0) wait2(0, &sh_known[2]);
     __syncthreads();
     if (sh_state < 0) return poison();
+    int known = sh_known[2];  // tiles k < known are published
     fetch(0);
     ktrsv::cp_commit();
     for (int k = 0; k < c; ++k) {
-      const bool more = k + 1 < c;
-      if (tid == 0)
-        sh_ready[k & 1] = more ? peek2(&flags[tidx(i, k + 1)], &flags[tidx(c, k + 1)]) : 0;
+      const bool more = k + 1 < c, ask = more && k + 1 >= known;
+      if (ask && warp == 0) scan(k + 1, &sh_known[k & 1]);
       ktrsv::cp_wait_all();
       __syncthreads();  // tile k landed; every thread is done with the other buffers
-      const bool ready = more && sh_ready[k & 1] > 0;
-      if (ready) fetch(k + 1);
+      if (ask) known = sh_known[k & 1];
+      const bool now = more && k + 1 < known;
+      if (now) fetch(k + 1);
       ktrsv::cp_commit();
       const T* Ak = A0 + (k & 1) * TILE;
       const T* Bk = B0 + (k & 1) * TILE;
-      if (!diag) product8<NB / G>(acc, Ak, Bk, grp * (NB / G), u);
+      if (!diag) product8<NB, NB, NB / G>(acc, Ak, Bk, grp * (NB / G), u);
       else
-        product8<2 * NB / G>(acc, Ak, grp < G / 2 ? Bk : Ak, (grp % (G / 2)) * (2 * NB / G), u);
-      if (more && !ready) {
-        if (tid == 0) sh_state = wait2(k + 1);
+        product8<NB, NB, 2 * NB / G>(acc, Ak, grp < G / 2 ? Bk : Ak, (grp % (G / 2)) * (2 * NB / G), u);
+      if (more && !now) {
+        if (warp == 0) wait2(k + 1, &sh_known[2]);
         __syncthreads();
         if (sh_state < 0) return poison();
+        known = sh_known[2];
         fetch(k + 1);
         ktrsv::cp_commit();
       }
@@ -486,24 +384,24 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
           store8(A0 + grp * TILE, acc, u);
         }
         __syncthreads();
-        subtract<4>(Ts, A0);
+        subtract<4, THR>(Ts, A0);
       } else {
         if (grp < 4) store8(A0 + grp * TILE, acc, u);
         __syncthreads();
-        subtract<4>(Ts, A0);
+        subtract<4, THR>(Ts, A0);
         __syncthreads();
         if (grp >= 4) store8(A0 + (grp - 4) * TILE, acc, u);
         __syncthreads();
-        subtract<4>(Ss, A0);
+        subtract<4, THR>(Ss, A0);
       }
     } else {
       store8(A0 + grp * TILE, acc, u);
       __syncthreads();
       if (!diag) {
-        subtract<4>(Ts, A0);
+        subtract<4, THR>(Ts, A0);
       } else {
-        subtract<2>(Ts, A0);
-        subtract<2>(Ss, A0 + 2 * TILE);
+        subtract<2, THR>(Ts, A0);
+        subtract<2, THR>(Ss, A0 + 2 * TILE);
       }
     }
   }

@@ -47,10 +47,9 @@ int trsm_rec(ExecT<T>& ex, ViewT<T> L, int n, ViewT<T> B, int m, Scalar<T> alpha
     p.inplace = 1;
     return ex.gemm(&p, 1);
   }
-  // Few right-hand sides: the whole block goes to the wavefront solve (its
-  // chain is short relative to the work).  Many right-hand sides: small
-  // leaves, so that most of the work is in the (tensor-core) GEMM updates.
-  if (n <= (m <= kTrsvMaxRhs * 4 ? kWaveLeaf : (math ? kWaveLeafWideTc : kWaveLeafWide))) {
+  // Leaves go to the wavefront solve, small ones, so that most of the work is
+  // in the (tensor-core) GEMM updates.
+  if (n <= kWaveLeaf) {
     int rc = ex.trsm_wave(L, n, B, m, alpha, Wb);
     if (rc != kNotSupported) return rc;
   }
@@ -74,9 +73,10 @@ int trsm_lln(ExecT<T>& ex, ViewT<T> L, int n, ViewT<T> B, int m, Scalar<T> alpha
   if (!W) return 2;
   int rc = ex.trtri_blocks(L, n, kTrsmLeaf, W);
   if (rc) return rc;
-  // One wavefront launch for few right-hand sides; with tensor-core updates
-  // available the recursive solve wins above kTrsvMaxRhsTc of them.
-  if (m <= (math ? kTrsvMaxRhsTc : kTrsvMaxRhs)) {
+  // One wavefront launch for few right-hand sides: up to kTrsvMaxRhs the
+  // recursion's launches cost more than its products save, tensor cores or not
+  // (n = 4096, 400 columns: 0.5 ms against 0.9 ms).
+  if (m <= kTrsvMaxRhs) {
     rc = ex.trsm_wave(L, n, B, m, alpha, W);
     if (rc != kNotSupported) return rc;
   }
@@ -101,14 +101,13 @@ int trsm(ExecT<T>& ex, int left, int lower, int trans, ViewT<T> Tm, ViewT<T> B, 
 template <typename T>
 int trmm_lln(ExecT<T>& ex, ViewT<T> L, int n, ViewT<T> B, int m, Scalar<T> alpha, int math) {
   if (n <= 0 || m <= 0) return 0;
-  int leaf = kTrmmLeaf < ex.inplace_rows() ? kTrmmLeaf : ex.inplace_rows();
-  if (n <= leaf) {
+  if (n <= ex.inplace_rows()) {
     GemmProbT<T> p = gemm_prob(L, B, B, n, m, n, alpha, 0.0f, 0);
     p.a_tri = 1;
     p.inplace = 1;
     return ex.gemm(&p, 1);
   }
-  int n1 = split(n, leaf), n2 = n - n1;
+  int n1 = split(n, kTriTile), n2 = n - n1;
   int rc = trmm_lln(ex, sub(L, n1, n1), n2, sub(B, n1, 0), m, alpha, math);
   if (rc) return rc;
   GemmProbT<T> p = gemm_prob(sub(L, n1, 0), B, sub(B, n1, 0), n2, m, n1, alpha,
@@ -156,7 +155,7 @@ int potrf_lower(ExecT<T>& ex, ViewT<T> A, int n, int info_base, int math) {
 template <typename T>
 int trtri_lower(ExecT<T>& ex, ViewT<T> L, int n, int math) {
   if (n <= 0) return 0;
-  if (n <= kTriTile) return ex.trtri_tile(L, n);
+  if (n <= ex.trtri_rows()) return ex.trtri_block(L, n);
   int n1 = split(n, kTriTile), n2 = n - n1;
   int rc = trtri_lower(ex, L, n1, math);
   if (rc) return rc;
@@ -170,7 +169,7 @@ int trtri_lower(ExecT<T>& ex, ViewT<T> L, int n, int math) {
 template <typename T>
 int lauum_lower(ExecT<T>& ex, ViewT<T> L, int n, int math) {
   if (n <= 0) return 0;
-  if (n <= kTriTile) return ex.lauum_tile(L, n);
+  if (n <= ex.lauum_rows()) return ex.lauum_block(L, n);
   int n1 = split(n, kTriTile), n2 = n - n1;
   ViewT<T> L21 = sub(L, n1, 0);
   int rc = lauum_lower(ex, L, n1, math);
