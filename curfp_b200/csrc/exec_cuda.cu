@@ -5,6 +5,7 @@
 #include <type_traits>
 
 #include "context.h"
+#include "k_chain.cuh"
 #include "k_chol.cuh"
 #include "k_gemm.cuh"
 #include "gemm_route.h"
@@ -553,12 +554,59 @@ int launch_wave(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int n, Vie
 }
 }  // namespace
 
-// Up to 8 right-hand sides: 8-column chunks (the per-block products of the
-// chain shrink with the chunk); otherwise 64-column chunks.
+namespace {
+// The solve whose chain runs inside clusters (k_chain.cuh), NC columns a chunk.
+template <typename T, int NC>
+int launch_chain(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int n, ViewT<T> B, int m,
+                 T alpha, const T* W) {
+  using C = kchain::Cfg<T, NC>;
+  kchain::Args<T> a{};
+  a.L = L; a.B = B;
+  a.n = n; a.m = m;
+  a.nblk = (n + kchain::NB - 1) / kchain::NB;
+  a.nchunk = (m + NC - 1) / NC;
+  a.alpha = alpha;
+  a.W = W;
+  const size_t tiles = (size_t)a.nblk * a.nchunk, words = 1 + tiles;
+  a.ws = static_cast<T*>(
+      grow_buffer(ctx, &ctx->wst, &ctx->wst_bytes, tiles * C::XT * sizeof(T)));
+  a.sync = static_cast<int*>(grow_buffer(ctx, &ctx->tsv, &ctx->tsv_bytes, words * sizeof(int)));
+  if (!a.ws || !a.sync) return 2;
+  if (cudaMemsetAsync(a.sync, 0, words * sizeof(int), ctx->stream) != cudaSuccess) return 4;
+  a.err = ctx->d_info + 1;
+  a.abort_flag = abort_flag;
+  static const bool attr = smem_attr(kchain::trsm_chain<T, NC>, C::SMEM);
+  if (!attr) return 4;
+  ProfScope ps(ctx->prof, ctx->stream, K_TRSV, (double)n * n * m, (double)n * n * sizeof(T) / 2.0);
+  ps.shape(n, m, n, (int)tiles);
+  const int grid = (a.nblk + kchain::CS - 1) / kchain::CS * a.nchunk * kchain::CS;
+  kchain::trsm_chain<T, NC><<<grid, kchain::THR, C::SMEM, ctx->stream>>>(a);
+  ++ctx->launches;
+  ++ctx->wait_launches;
+  return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+}  // namespace
+
+// Up to kTrsvMaxRhs right-hand sides (FP64 128): the chain inside clusters, in
+// chunks as narrow as the throughput allows, since the chain's step shrinks
+// with the chunk while the products' cost per column grows: 8 columns up to
+// 256 (block row, chunk) pairs, 16 up to 512, else 32 (8192 rows, 16 / 64 / 128
+// columns: 8 wide 190 / 510 / 970 us, 16 wide 262 / 390 / 690 us, 32 wide 400 /
+// 420 / 600 us; FP64 8 wide).  More right-hand sides keep every SM busy:
+// 64-column chunks handed on through L2 (n = 512 leaves of the recursion).
 template <typename T>
 int CudaExecT<T>::trsm_wave(ViewT<T> L, int n, ViewT<T> B, int m, T alpha, const T* W) {
   if (n <= 0 || m <= 0) return 0;
-  if (m <= 8) return launch_wave<T, 8>(ctx_, abort_, L, n, B, m, alpha, W);
+  const int nblk = (n + kTrsmLeaf - 1) / kTrsmLeaf;
+  if (m <= (sizeof(T) == 4 ? kTrsvMaxRhs : 128)) {
+    if constexpr (sizeof(T) == 4) {
+      if ((int64_t)nblk * ((m + 15) / 16) > 512)
+        return launch_chain<T, 32>(ctx_, abort_, L, n, B, m, alpha, W);
+      if ((int64_t)nblk * ((m + 7) / 8) > 256)
+        return launch_chain<T, 16>(ctx_, abort_, L, n, B, m, alpha, W);
+    }
+    return launch_chain<T, 8>(ctx_, abort_, L, n, B, m, alpha, W);
+  }
   return launch_wave<T, 64>(ctx_, abort_, L, n, B, m, alpha, W);
 }
 
