@@ -93,6 +93,10 @@ class CudaExecT : public ExecT<T> {
                 int math) override;
   int trsm_wave(ViewT<T> L, int n, ViewT<T> B, int m, T alpha, const T* W) override;
   int potrf_adj_tile(ViewT<T> L, ViewT<T> G, int n) override;
+  // Whether products may take scratch for split sums from the workspaces.
+  virtual bool may_allocate() const { return true; }
+  bool batch_inverses() const override { return may_allocate(); }
+  int trtri_batch(const ViewT<T>* L, const int* n, int count, T* W) override;
   // When set, work after the first diagonal block waits for this event.
   int after_first_block() override {
     if (!rest_ready) return 0;

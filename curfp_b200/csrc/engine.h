@@ -111,6 +111,13 @@ class ExecT {
   // written to W + b*nb*nb, column-major with ld nb, zeros above the diagonal.
   // (W: nblk records of kInvStride floats, see kInvStride)
   virtual int trtri_blocks(ViewT<T> L, int n, int nb, T* W) = 0;
+  // trtri_blocks of several matrices into consecutive records from W on, as one
+  // operation, for executors with batch_inverses().
+  virtual bool batch_inverses() const { return false; }
+  virtual int trtri_batch(const ViewT<T>* L, const int* n, int count, T* W) {
+    (void)L; (void)n; (void)count; (void)W;
+    return kNotSupported;
+  }
   // In-place inverse of lower L (n <= kTriTile).
   virtual int trtri_tile(ViewT<T> L, int n) = 0;
   // In-place L := L^T L (lower triangle; n <= kTriTile).

@@ -1,5 +1,6 @@
 // exec_cuda.cu — CUDA executor: turns planner primitives into sm_100a kernel
 // launches on the handle's stream.
+#include <algorithm>
 #include <climits>
 #include <cstdint>
 #include <type_traits>
@@ -50,7 +51,7 @@ namespace {
 
 template <typename T, int BM, int BN>
 int launch_gemm(const GemmProbT<T>* p, int count, const int* abort_flag,
-                curfpContext* ctx) {
+                curfpContext* ctx, bool alloc = false) {
   cudaStream_t st = ctx->stream;
   double flops = 0;
   kgemm::Batch<T> b{};
@@ -82,25 +83,58 @@ int launch_gemm(const GemmProbT<T>* p, int count, const int* abort_flag,
   b.count = cnt;
   b.total_tiles = tiles;
   b.abort_flag = abort_flag;
+  // One unmasked product with few tiles and a long k (the solves' rectangle
+  // updates): k is split so that about two CTAs per SM run, their partial
+  // tiles added in order by split_reduce (2048 x 64, k = 2048: 32 CTAs 170 us,
+  // with the split 60 us).
+  int splits = 1;
+  const kgemm::Prob<T>& q0 = b.p[0];
+  if (alloc && cnt == 1 && !q0.k2 && !q0.a_tri && !q0.b_tri && !q0.c_lower && !p[0].inplace) {
+    splits = std::min(2 * 148 / tiles, q0.k / 128);
+    if (splits < 2) splits = 1;
+    b.kseg = ((q0.k + splits - 1) / splits + 31) / 32 * 32;
+    splits = (q0.k + b.kseg - 1) / b.kseg;
+  }
+  if (splits > 1) {
+    b.part = static_cast<T*>(grow_buffer(ctx, &ctx->wst, &ctx->wst_bytes,
+                                         (size_t)splits * tiles * BM * BN * sizeof(T)));
+    if (!b.part) return 2;
+  }
   ProfScope ps(ctx->prof, st, K_SGEMM, flops, 0);
   ps.shape(b.p[0].m, b.p[0].n, b.p[0].k + b.p[0].k2, tiles);
-  kgemm::sgemm_batch<T, BM, BN><<<tiles, kgemm::kThreads, 0, st>>>(b);
+  kgemm::sgemm_batch<T, BM, BN><<<dim3(tiles, splits), kgemm::kThreads, 0, st>>>(b);
   ++ctx->launches;
+  if (splits > 1) {
+    kgemm::split_reduce<T, BM, BN><<<tiles, kgemm::kThreads, 0, st>>>(b, splits);
+    ++ctx->launches;
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
 // The few-column kernels (k_skinny.cuh) for the products gemm_route.h
 // routes to them; -1 when it does not.
 template <typename T>
-int launch_skinny(const GemmProbT<T>& g0, const int* abort_flag, curfpContext* ctx) {
+int launch_skinny(const GemmProbT<T>& g0, const int* abort_flag, curfpContext* ctx, bool alloc) {
   GemmProbT<T> g;
   const SkinnyRoute r = skinny_route(g0, &g);
   if (!r.use) return -1;
-  const kskinny::Args<T> a{g.A.p, g.A.rs, g.A.cs, g.B.p, g.B.rs, g.B.cs, g.C.p, g.C.rs, g.C.cs,
-                           g.m, g.n, g.k, g.alpha, g.beta};
+  kskinny::Args<T> a{g.A.p, g.A.rs, g.A.cs, g.B.p, g.B.rs, g.B.cs, g.C.p, g.C.rs, g.C.cs,
+                     g.m, g.n, g.k, g.alpha, g.beta, g.k, nullptr};
   ProfScope ps(ctx->prof, ctx->stream, K_SGEMM, 2.0 * g.m * g.n * (double)g.k,
                (double)sizeof(T) * g.m * (double)g.k);
-  const int grid = (g.m + 31) / 32;
+  // about eight CTAs per SM, at least 512 columns each
+  int splits = 1;
+  if (alloc) {
+    splits = (int)std::min<int64_t>((int64_t)8 * 148 * 32 / g.m + 1, (g.k + 511) / 512);
+    a.kseg = ((g.k + splits - 1) / splits + 31) / 32 * 32;
+    splits = (g.k + a.kseg - 1) / a.kseg;
+  }
+  if (splits > 1) {
+    a.part = static_cast<T*>(grow_buffer(ctx, &ctx->wst, &ctx->wst_bytes,
+                                         (size_t)splits * g.n * g.m * sizeof(T)));
+    if (!a.part) return 2;
+  }
+  const dim3 grid((g.m + 31) / 32, splits);
   cudaStream_t st = ctx->stream;
   auto go = [&](auto ncols) {
     constexpr int N = decltype(ncols)::value;
@@ -114,6 +148,11 @@ int launch_skinny(const GemmProbT<T>& g0, const int* abort_flag, curfpContext* c
     default: go(std::integral_constant<int, 8>{}); break;
   }
   ++ctx->launches;
+  if (splits > 1) {
+    kskinny::skinny_reduce<T><<<dim3((g.m + kskinny::kThreads - 1) / kskinny::kThreads, g.n),
+                                kskinny::kThreads, 0, st>>>(a, splits, abort_flag);
+    ++ctx->launches;
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
@@ -261,7 +300,7 @@ int CudaExecT<double>::gemm(const GemmProbT<double>* p, int count) {
   if (count <= 0) return 0;
   if (count > kMaxBatch) return 3;
   if (count == 1) {
-    const int rc = launch_skinny<double>(p[0], abort_, ctx_);
+    const int rc = launch_skinny<double>(p[0], abort_, ctx_, may_allocate());
     if (rc >= 0) return rc;
   }
   GemmProbT<double> q;
@@ -281,7 +320,7 @@ int CudaExecT<double>::gemm(const GemmProbT<double>* p, int count) {
     inplace = inplace || p[i].inplace;
   }
   if (t128 >= 148 && !inplace) return launch_gemm<double, 128, 128>(p, count, abort_, ctx_);
-  return launch_gemm<double, 64, 64>(p, count, abort_, ctx_);
+  return launch_gemm<double, 64, 64>(p, count, abort_, ctx_, may_allocate());
 }
 
 template <>
@@ -289,7 +328,7 @@ int CudaExecT<float>::gemm(const GemmProb* p, int count) {
   if (count <= 0) return 0;
   if (count > kMaxBatch) return 3;
   if (count == 1) {
-    const int rc = launch_skinny<float>(p[0], abort_, ctx_);
+    const int rc = launch_skinny<float>(p[0], abort_, ctx_, may_allocate());
     if (rc >= 0) return rc;
   }
   // One problem, one or two products, on the tensor cores: the A operands
@@ -337,7 +376,7 @@ int CudaExecT<float>::gemm(const GemmProb* p, int count) {
   }
   if (t128 >= 2 * 148 && maxm == 0)
     return launch_gemm<float, 128, 128>(p, count, abort_, ctx_);
-  return launch_gemm<float, 64, 64>(p, count, abort_, ctx_);
+  return launch_gemm<float, 64, 64>(p, count, abort_, ctx_, may_allocate());
 }
 
 namespace {
@@ -424,32 +463,42 @@ int CudaExecT<T>::potrf_panel(ViewT<T> L, ViewT<T> A21, int n1, int n2, int info
 }
 
 template <typename T>
-int CudaExecT<T>::trtri_blocks(ViewT<T> L, int n, int nb, T* W) {
-  if (n <= 0) return 0;
-  if (nb != ktile::T) return 3;
-  int nblk = (n + nb - 1) / nb;
-  ProfScope ps(ctx_->prof, ctx_->stream, K_TRTRI, (double)n * nb * nb / 3.0, 0);
+int CudaExecT<T>::trtri_batch(const ViewT<T>* L, const int* n, int count, T* W) {
+  ktile::TriBatch<T> b{};
+  if (count > ktile::TriBatch<T>::MAX) return 3;
+  int blocks = 0;
+  double flops = 0;
+  for (int i = 0; i < count; ++i) {
+    b.L[i] = L[i];
+    b.n[i] = n[i];
+    b.begin[i] = blocks;
+    blocks += n[i] > 0 ? (n[i] + ktile::T - 1) / ktile::T : 0;
+    flops += (double)n[i] * ktile::T * ktile::T / 3.0;
+  }
+  if (blocks == 0) return 0;
+  b.count = count;
+  b.W = W;
+  ProfScope ps(ctx_->prof, ctx_->stream, K_TRTRI, flops, 0);
   constexpr int smem = ktile::trtri_smem<T>();
   static const bool attr = smem_attr(ktile::trtri_blocks<T>, smem);
   if (!attr) return 4;
-  ktile::trtri_blocks<T>
-      <<<nblk, ktile::TRTRI_THREADS, smem, ctx_->stream>>>(L, n, W, abort_);
+  ktile::trtri_blocks<T><<<blocks, ktile::TRTRI_THREADS, smem, ctx_->stream>>>(b, abort_);
   ++ctx_->launches;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+
+template <typename T>
+int CudaExecT<T>::trtri_blocks(ViewT<T> L, int n, int nb, T* W) {
+  if (n <= 0) return 0;
+  if (nb != ktile::T) return 3;
+  return trtri_batch(&L, &n, 1, W);
 }
 
 template <typename T>
 int CudaExecT<T>::trtri_tile(ViewT<T> L, int n) {
   if (n <= 0) return 0;
   if (n > ktile::T) return 3;
-  ProfScope ps(ctx_->prof, ctx_->stream, K_TRTRI, (double)n * n * n / 3.0, 0);
-  constexpr int smem = ktile::trtri_smem<T>();
-  static const bool attr = smem_attr(ktile::trtri_blocks<T>, smem);
-  if (!attr) return 4;
-  ktile::trtri_blocks<T>
-      <<<1, ktile::TRTRI_THREADS, smem, ctx_->stream>>>(L, n, nullptr, abort_);
-  ++ctx_->launches;
-  return cudaGetLastError() == cudaSuccess ? 0 : 4;
+  return trtri_batch(&L, &n, 1, nullptr);
 }
 
 template <typename T>

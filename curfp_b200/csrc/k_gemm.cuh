@@ -52,6 +52,10 @@ struct Batch {
   int count;
   int total_tiles;
   const int* abort_flag;  // if non-null and *abort_flag != INT_MAX: no-op
+  // gridDim.y > 1 (one unmasked product): split y sums k in [y kseg, + kseg)
+  // into part, tiles of BM x BN row-major, which split_reduce adds in order.
+  int kseg;
+  T* part;
 };
 
 // Map a linear tile index of a problem to (ti, tj), in the L2-friendly
@@ -291,6 +295,13 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && BM >= 128) ? 1 : 
   int kb1, ke1, kb2, ke2;
   k_range<BK>(P.k, P.a_tri, P.b_tri, m0, n0, BM, BN, kb1, ke1);
   k_range<BK>(P.k2, P.a2_tri, P.b2_tri, m0, n0, BM, BN, kb2, ke2);
+  // only the 64 x 64 tiles are split (the 128 x 128 ones fill the machine)
+  const bool split = BM == 64 && gridDim.y > 1;
+  if (split) {  // kseg is a multiple of BK
+    kb1 = blockIdx.y * batch.kseg;
+    ke1 = min(ke1, kb1 + batch.kseg);
+  }
+  const int kd1 = split ? ke1 : P.k;  // depth that loads may read up to
   const int kt1 = (ke1 - kb1 + BK - 1) / BK;
   const int kt2 = (ke2 - kb2 + BK - 1) / BK;
   const int ktiles = kt1 + kt2;
@@ -300,8 +311,8 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && BM >= 128) ? 1 : 
   auto load = [&](int kt) {
     if (kt < kt1) {
       const int k0 = kb1 + kt * BK;
-      stage_load<T, BM, BK>(ra, P.A, P.a_rs, P.a_cs, P.m, P.k, P.a_tri, fl & 3, m0, k0);
-      stage_load<T, BN, BK>(rb, P.B, P.b_cs, P.b_rs, P.n, P.k, bcode(P.b_tri), (fl >> 2) & 3, n0,
+      stage_load<T, BM, BK>(ra, P.A, P.a_rs, P.a_cs, P.m, kd1, P.a_tri, fl & 3, m0, k0);
+      stage_load<T, BN, BK>(rb, P.B, P.b_cs, P.b_rs, P.n, kd1, bcode(P.b_tri), (fl >> 2) & 3, n0,
                             k0);
     } else {
       const int k0 = kb2 + (kt - kt1) * BK;
@@ -414,6 +425,8 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && BM >= 128) ? 1 : 
 
   // Epilogue.
   const T alpha = P.alpha, beta = P.beta;
+  T* const part =
+      split ? batch.part + ((int64_t)blockIdx.y * batch.total_tiles + t) * (BM * BN) : nullptr;
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
     const int gi = m0 + (i / 4) * (BM / GM) + tr * 4 + (i % 4);
@@ -424,11 +437,39 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && BM >= 128) ? 1 : 
                                     : n0 + (j / 4) * (BN / GN) + tc * 4 + (j % 4);
       if (gj >= P.n) continue;
       if (P.c_lower && gj > gi) continue;
+      if (BM == 64 && part) {
+        part[(gi - m0) * BN + gj - n0] = acc[i][j];
+        continue;
+      }
       T* c = P.C + (int64_t)gi * P.c_rs + (int64_t)gj * P.c_cs;
       T v = alpha * acc[i][j];
       if (beta != T(0)) v = fma(beta, *c, v);
       *c = v;
     }
+  }
+}
+
+// C := alpha (the splits' partial tiles, added in order) + beta C; one CTA per
+// tile of the single problem.
+template <typename T, int BM, int BN>
+__global__ void __launch_bounds__(kThreads) split_reduce(const Batch<T> batch, int splits) {
+  if (batch.abort_flag && *batch.abort_flag != INT_MAX) return;
+  const Prob<T>& P = batch.p[0];
+  int ti, tj;
+  tile_coords(P, blockIdx.x, ti, tj);
+  const bool rowcont = P.c_cs == 1 || P.c_cs == -1;
+  const T* part = batch.part + (int64_t)blockIdx.x * (BM * BN);
+  const int64_t step = (int64_t)batch.total_tiles * (BM * BN);
+  for (int e = threadIdx.x; e < BM * BN; e += kThreads) {
+    const int i = rowcont ? e / BN : e % BM, j = rowcont ? e % BN : e / BM;
+    const int gi = ti * BM + i, gj = tj * BN + j;
+    if (gi >= P.m || gj >= P.n) continue;
+    T s = part[i * BN + j];
+    for (int y = 1; y < splits; ++y) s += part[y * step + i * BN + j];
+    T* c = P.C + (int64_t)gi * P.c_rs + (int64_t)gj * P.c_cs;
+    T v = P.alpha * s;
+    if (P.beta != T(0)) v = fma(P.beta, *c, v);
+    *c = v;
   }
 }
 

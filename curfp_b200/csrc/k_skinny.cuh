@@ -5,11 +5,14 @@
 //
 // Bandwidth-bound: A (an RFP rectangle of up to n^2/4 elements) is read once,
 // along its contiguous dimension, with many independent loads in flight per
-// thread; B (k x N) is small and is re-read from L1/L2.  There is no split
-// of k across CTAs, so no partial sums leave the CTA and nothing is
-// allocated: each output element is summed in a fixed order (registers, then
-// a fixed-order combine through shared memory or warp shuffles), so the
-// result is bitwise repeatable.
+// thread; B (k x N) is small and is re-read from L1/L2.  k is split over
+// gridDim.y CTAs whose partial sums part[(y, c, i)] skinny_reduce adds in
+// order, so that several CTAs per SM keep loads in flight (8192 x 8192, one
+// column: 256 CTAs without the split 138 us, with it 70 us); gridDim.y = 1
+// writes C directly and needs no scratch (the no-allocation solve).  Every
+// element is summed in a fixed order (registers, then a fixed-order combine
+// through shared memory or warp shuffles, then the splits), so the result is
+// bitwise repeatable.
 //
 //  * skinny_rows (A's row index is the unit-stride one): a CTA owns 32 rows,
 //    lane = row; its 8 warps take interleaved blocks of U columns kk; the 8
@@ -34,10 +37,16 @@ struct Args {
   T* C; int64_t c_rs, c_cs;
   int m, n, k;  // n <= N of the instantiation (columns past n are neither read nor written)
   T alpha, beta;
+  int kseg;  // columns of A per split (a multiple of 32)
+  T* part;   // partial sums of the splits (gridDim.y > 1)
 };
 
 template <typename T>
 __device__ __forceinline__ void store_out(const Args<T>& a, int i, int c, T s) {
+  if (gridDim.y > 1) {
+    a.part[((int64_t)blockIdx.y * a.n + c) * a.m + i] = s;
+    return;
+  }
   T* p = a.C + (int64_t)i * a.c_rs + (int64_t)c * a.c_cs;
   *p = a.beta == T(0) ? a.alpha * s : fma(a.beta, *p, a.alpha * s);
 }
@@ -60,16 +69,17 @@ __global__ void __launch_bounds__(kThreads) skinny_rows(const Args<T> a, const i
     for (int c = 0; c < N; ++c)
       if (c < a.n) acc[c] = fma(av, __ldg(bk + (int64_t)c * a.b_cs), acc[c]);
   };
-  int k0 = w * U;
-  for (; k0 + U <= a.k; k0 += 8 * U) {
+  const int kb = blockIdx.y * a.kseg, ke = min(a.k, kb + a.kseg);
+  int k0 = kb + w * U;
+  for (; k0 + U <= ke; k0 += 8 * U) {
     T av[U];
 #pragma unroll
     for (int t = 0; t < U; ++t) av[t] = __ldg(Ai + (int64_t)(k0 + t) * a.a_cs);
 #pragma unroll
     for (int t = 0; t < U; ++t) step(k0 + t, av[t]);
   }
-  if (k0 < a.k)
-    for (int t = 0; k0 + t < a.k; ++t) step(k0 + t, __ldg(Ai + (int64_t)(k0 + t) * a.a_cs));
+  if (k0 < ke)
+    for (int t = 0; k0 + t < ke; ++t) step(k0 + t, __ldg(Ai + (int64_t)(k0 + t) * a.a_cs));
   __shared__ T part[8][N][32];
 #pragma unroll
   for (int c = 0; c < N; ++c) part[w][c][lane] = acc[c];
@@ -104,12 +114,13 @@ __global__ void __launch_bounds__(kThreads) skinny_cols(const Args<T> a, const i
   for (int r = 0; r < RW; ++r)
 #pragma unroll
     for (int c = 0; c < N; ++c) acc[r][c] = T(0);
+  const int kb = blockIdx.y * a.kseg, ke = min(a.k, kb + a.kseg);
   auto block = [&](int k0, bool guard) {
     T av[U][RW], bv[U][N];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int kk = k0 + 32 * u + lane;
-      const bool kok = !guard || kk < a.k;
+      const bool kok = !guard || kk < ke;
 #pragma unroll
       for (int r = 0; r < RW; ++r) av[u][r] = kok ? __ldg(Ar[r] + (int64_t)kk * a.a_cs) : T(0);
 #pragma unroll
@@ -124,9 +135,9 @@ __global__ void __launch_bounds__(kThreads) skinny_cols(const Args<T> a, const i
 #pragma unroll
         for (int c = 0; c < N; ++c) acc[r][c] = fma(av[u][r], bv[u][c], acc[r][c]);
   };
-  int k0 = 0;
-  for (; k0 + 32 * U <= a.k; k0 += 32 * U) block(k0, false);
-  if (k0 < a.k) block(k0, true);
+  int k0 = kb;
+  for (; k0 + 32 * U <= ke; k0 += 32 * U) block(k0, false);
+  if (k0 < ke) block(k0, true);
 #pragma unroll
   for (int r = 0; r < RW; ++r)
 #pragma unroll
@@ -144,6 +155,19 @@ __global__ void __launch_bounds__(kThreads) skinny_cols(const Args<T> a, const i
         for (int c = 0; c < N; ++c)
           if (c < a.n) store_out(a, i0 + r, c, acc[r][c]);
   }
+}
+
+// C := alpha (the splits' partial sums, added in order) + beta C.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) skinny_reduce(const Args<T> a, int splits,
+                                                          const int* abort_flag) {
+  if (abort_flag && *abort_flag != INT_MAX) return;
+  const int i = blockIdx.x * kThreads + threadIdx.x, c = blockIdx.y;
+  if (i >= a.m) return;
+  T s = a.part[(int64_t)c * a.m + i];
+  for (int y = 1; y < splits; ++y) s += a.part[((int64_t)y * a.n + c) * a.m + i];
+  T* p = a.C + (int64_t)i * a.c_rs + (int64_t)c * a.c_cs;
+  *p = a.beta == T(0) ? a.alpha * s : fma(a.beta, *p, a.alpha * s);
 }
 
 }  // namespace kskinny

@@ -67,9 +67,11 @@ static_assert(T == kTrsmLeaf && T == kTriTile, "tile kernels assume one tile siz
 
 // Inverse of lower-triangular diagonal blocks.  Block b = blockIdx.x covers
 // rows/cols [b*64, min(n, b*64+64)); 256 threads.  The two 32 x 32 diagonal
-// quarters are inverted in registers by warps 0 and 1 (lane = row, right-
-// looking: row j of the inverse is final once scaled by 1/D_jj, then is
-// broadcast to the rows below), and the off-diagonal quarter follows as
+// quarters are inverted in registers by warps 0 and 1 (lane = column of the
+// inverse, right-looking: element j is final once scaled by 1/D_jj, then
+// updates the elements below with broadcast reads of D's column; by row and
+// shuffle a launch took 20 us, so 18 us for four matrices), and the off-diagonal quarter
+// follows as
 // inv([D0 0; B D1]) = [inv(D0) 0; -inv(D1) (B inv(D0))  inv(D1)] by two
 // 32 x 32 products over all threads.  W != nullptr: block b writes the record
 // W + b*kInvStride = [W_b | M_b], both 64 x 64 column-major (ld 64, zeros
@@ -81,14 +83,30 @@ constexpr int TRTRI_THREADS = 256;
 template <typename E>
 constexpr int trtri_smem() { return 2 * T * LD * (int)sizeof(E); }
 
+// Several matrices in one launch: matrix i's blocks are begin[i] .. of the
+// grid, and their records follow each other at W.
 template <typename E>
-__global__ void __launch_bounds__(TRTRI_THREADS) trtri_blocks(ViewT<E> L, int n, E* W,
+struct TriBatch {
+  static constexpr int MAX = 4;
+  ViewT<E> L[MAX];
+  int n[MAX], begin[MAX], count;
+  E* W;
+};
+
+template <typename E>
+__global__ void __launch_bounds__(TRTRI_THREADS) trtri_blocks(const TriBatch<E> batch,
                                                               const int* abort_flag) {
   if (abort_flag && *abort_flag != INT_MAX) return;
+  int mi = 0;
+  while (mi + 1 < batch.count && (int)blockIdx.x >= batch.begin[mi + 1]) ++mi;
+  const ViewT<E> L = batch.L[mi];
+  const int n = batch.n[mi];
+  E* const W = batch.W ? batch.W + (int64_t)batch.begin[mi] * kInvStride : nullptr;
   extern __shared__ __align__(16) unsigned char trtri_raw[];
+  __shared__ E rinv[T];
   E (*s)[LD] = reinterpret_cast<E (*)[LD]>(trtri_raw);  // L_bb, later the block left of it
   E (*x)[LD] = s + T;  // the inverse (upper-right quarter: scratch)
-  const int b = blockIdx.x, r0 = b * T;
+  const int b = blockIdx.x - batch.begin[mi], r0 = b * T;
   const int sz = min(T, n - r0);
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   const ViewT<E> Lb = sub(L, r0, r0);
@@ -101,31 +119,21 @@ __global__ void __launch_bounds__(TRTRI_THREADS) trtri_blocks(ViewT<E> L, int n,
   __syncthreads();
   load_lower<LD>(Lb, sz, &s[0][0]);
   __syncthreads();
+  if (tid < T) rinv[tid] = tid < sz ? E(1) / s[tid][tid] : E(0);
+  __syncthreads();
   if (warp < 2) {
-    const int q0 = warp * 32, w = min(32, sz - q0);
-    if (w > 0) {
-      E a[32], xr[32];
+    const int q0 = warp * 32;
+    E xc[32];
 #pragma unroll
-      for (int k = 0; k < 32; ++k) {
-        a[k] = (lane < w && k <= lane) ? s[q0 + lane][q0 + k] : E(0);
-        xr[k] = (k == lane && lane < w) ? E(1) : E(0);
-      }
-      const E rl = lane < w ? E(1) / s[q0 + lane][q0 + lane] : E(0);
+    for (int k = 0; k < 32; ++k) xc[k] = k == lane && q0 + lane < sz ? E(1) : E(0);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        if (j < w) {
-          const E sc = lane == j ? rl : E(1);
+    for (int j = 0; j < 32; ++j) {
+      xc[j] *= rinv[q0 + j];
 #pragma unroll
-          for (int k = 0; k <= j; ++k) {
-            xr[k] *= sc;
-            const E v = __shfl_sync(0xffffffffu, xr[k], j);
-            if (lane > j) xr[k] = fma(-a[j], v, xr[k]);
-          }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 32; ++k) x[q0 + lane][q0 + k] = xr[k];
+      for (int k = j + 1; k < 32; ++k) xc[k] = fma(-s[q0 + k][q0 + j], xc[j], xc[k]);
     }
+#pragma unroll
+    for (int k = 0; k < 32; ++k) x[q0 + k][q0 + lane] = xc[k];
   }
   __syncthreads();
   if (sz > 32) {

@@ -85,6 +85,8 @@ class NoAllocExec : public rfp::CudaExec {
     return nfloats <= kInvFloats ? scratch_ : nullptr;
   }
 
+  bool may_allocate() const override { return false; }
+
   int trsm_wave(rfp::View L, int n, rfp::View B, int m, float alpha,
                 const float* W) override {
     int* sync = reinterpret_cast<int*>(scratch_ + kInvFloats);

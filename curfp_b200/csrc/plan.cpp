@@ -65,14 +65,22 @@ int trsm_rec(ExecT<T>& ex, ViewT<T> L, int n, ViewT<T> B, int m, Scalar<T> alpha
 
 }  // namespace
 
+namespace {
+inline int inv_blocks(int n) { return (n + kTrsmLeaf - 1) / kTrsmLeaf; }
+
+// L X = alpha B with the records of L's diagonal blocks at W; W == nullptr:
+// they are formed here.
 template <typename T>
-int trsm_lln(ExecT<T>& ex, ViewT<T> L, int n, ViewT<T> B, int m, Scalar<T> alpha, int math) {
+int trsm_with(ExecT<T>& ex, ViewT<T> L, int n, ViewT<T> B, int m, Scalar<T> alpha, int math,
+              const T* W) {
   if (n <= 0 || m <= 0) return 0;
-  int nblk = (n + kTrsmLeaf - 1) / kTrsmLeaf;
-  T* W = ex.workspace((size_t)nblk * kInvStride);
-  if (!W) return 2;
-  int rc = ex.trtri_blocks(L, n, kTrsmLeaf, W);
-  if (rc) return rc;
+  int rc;
+  if (!W) {
+    T* w = ex.workspace((size_t)inv_blocks(n) * kInvStride);
+    if (!w) return 2;
+    if ((rc = ex.trtri_blocks(L, n, kTrsmLeaf, w))) return rc;
+    W = w;
+  }
   // One wavefront launch for few right-hand sides: up to kTrsvMaxRhs the
   // recursion's launches cost more than its products save, tensor cores or not
   // (n = 4096, 400 columns: 0.5 ms against 0.9 ms).
@@ -81,6 +89,12 @@ int trsm_lln(ExecT<T>& ex, ViewT<T> L, int n, ViewT<T> B, int m, Scalar<T> alpha
     if (rc != kNotSupported) return rc;
   }
   return trsm_rec(ex, L, n, B, m, alpha, W, 0, math);
+}
+}  // namespace
+
+template <typename T>
+int trsm_lln(ExecT<T>& ex, ViewT<T> L, int n, ViewT<T> B, int m, Scalar<T> alpha, int math) {
+  return trsm_with<T>(ex, L, n, B, m, alpha, math, nullptr);
 }
 
 template <typename T>
@@ -261,20 +275,37 @@ int spftrs(ExecT<T>& ex, int transr, int lower, int n, int nrhs, const T* A,
   ViewT<T> B1{B, 1, ldb};
   ViewT<T> B2 = sub(B1, g.n1, 0);
   int rc;
+  // The four triangular solves in canonical form (trsm): L11, L22, then their
+  // transposes reversed; their diagonal blocks' records in one launch.
+  const ViewT<T> R22 = rev(tr(V22), g.n2, g.n2), R11 = rev(tr(V11), g.n1, g.n1);
+  const T* W[4] = {nullptr, nullptr, nullptr, nullptr};
+  if (ex.batch_inverses()) {
+    const ViewT<T> L[4] = {V11, V22, R22, R11};
+    const int sz[4] = {g.n1, g.n2, g.n2, g.n1};
+    size_t at[4], total = 0;
+    for (int i = 0; i < 4; ++i) {
+      at[i] = total;
+      total += (size_t)inv_blocks(sz[i]) * kInvStride;
+    }
+    T* w = ex.workspace(total);
+    if (!w) return 2;
+    if ((rc = ex.trtri_batch(L, sz, 4, w))) return rc;
+    for (int i = 0; i < 4; ++i) W[i] = w + at[i];
+  }
   // Forward: L Y = B.
-  if ((rc = trsm_lln(ex, V11, g.n1, B1, nrhs, 1.0f, math))) return rc;
+  if ((rc = trsm_with<T>(ex, V11, g.n1, B1, nrhs, 1.0f, math, W[0]))) return rc;
   if (g.n1 > 0 && g.n2 > 0) {
     GemmProbT<T> p = gemm_prob(V21, B1, B2, g.n2, nrhs, g.n1, -1.0f, 1.0f, math);
     if ((rc = ex.gemm(&p, 1))) return rc;
   }
-  if ((rc = trsm_lln(ex, V22, g.n2, B2, nrhs, 1.0f, math))) return rc;
+  if ((rc = trsm_with<T>(ex, V22, g.n2, B2, nrhs, 1.0f, math, W[1]))) return rc;
   // Backward: L^T X = Y.
-  if ((rc = trsm(ex, 1, 1, 1, V22, B2, g.n2, nrhs, 1.0f, math))) return rc;
+  if ((rc = trsm_with<T>(ex, R22, g.n2, rev_rows(B2, g.n2), nrhs, 1.0f, math, W[2]))) return rc;
   if (g.n1 > 0 && g.n2 > 0) {
     GemmProbT<T> p = gemm_prob(tr(V21), B2, B1, g.n1, nrhs, g.n2, -1.0f, 1.0f, math);
     if ((rc = ex.gemm(&p, 1))) return rc;
   }
-  return trsm(ex, 1, 1, 1, V11, B1, g.n1, nrhs, 1.0f, math);
+  return trsm_with<T>(ex, R11, g.n1, rev_rows(B1, g.n1), nrhs, 1.0f, math, W[3]);
 }
 
 template <typename T>
