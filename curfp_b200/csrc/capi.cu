@@ -14,6 +14,7 @@
 #include "k_pack.cuh"
 #include "k_refine.cuh"
 #include "k_symv.cuh"
+#include "k_symv2.cuh"
 #include "status.cuh"
 
 using rfp::CudaExec;
@@ -620,6 +621,21 @@ static curfpStatus_t sfmv_impl(curfpHandle_t handle, curfpOperation_t transr,
     return status_of(rfp::plan::rfp_symm(ex, tr, lower, n, arf, X, Y, 1, *alpha, *beta));
   }
   const Geometry g = rfp::geometry(n, tr, lower);
+  if constexpr (sizeof(T) == 4) {
+    rfp::ksymv2::Args a{};
+    const int64_t total = rfp::ksymv2::plan(g, &a);
+    float* part = static_cast<float*>(rfp::grow_buffer(handle, &handle->ws, &handle->ws_bytes,
+                                                       (size_t)total * sizeof(float)));
+    if (!part) return CURFP_STATUS_ALLOC_FAILED;
+    const double nt = (double)n * (n + 1) / 2;
+    rfp::ProfScope ps(handle->prof, handle->stream, rfp::K_SGEMM, 4.0 * nt, sizeof(T) * nt);
+    rfp::ksymv2::symv2_strips<<<dim3(a.groups, a.strips), rfp::ksymv2::THR, 0, handle->stream>>>(
+        a, arf, x + ox, incx, part);
+    rfp::ksymv2::symv2_reduce<<<(n + 31) / 32, rfp::ksymv2::THR, 0, handle->stream>>>(
+        a, part, y + oy, incy, *alpha, *beta);
+    handle->launches += 2;
+    return ok_launch() ? CURFP_STATUS_SUCCESS : CURFP_STATUS_EXECUTION_FAILED;
+  }
   const rfp::ksymv::Parts P = rfp::ksymv::parts(n);
   T* part = static_cast<T*>(rfp::grow_buffer(handle, &handle->ws, &handle->ws_bytes,
                                              (size_t)(P.n_row + P.n_col) * sizeof(T)));
