@@ -381,8 +381,9 @@ def stfttr(arf: torch.Tensor, *, transr: str = "T", uplo: str = "U",
     _validate(arf, "arf")
     if n is None:
         n = _n_from_rfp(arf.numel())
-    A = torch.zeros(n, n, dtype=torch.float32, device=arf.device)
-    stfttr_raw(_get_handle(), _op(transr), _fill(uplo), n, arf, A, n)
+    A = torch.empty(n, n, dtype=torch.float32, device=arf.device)
+    h = _get_handle()
+    check(h._lib.curfpSstfttrFill(h.ptr, _op(transr), _fill(uplo), n, _ptr(arf), _ptr(A), n))
     return A
 
 

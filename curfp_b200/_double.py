@@ -233,12 +233,13 @@ def dstrttf(A: torch.Tensor, *, transr: str = "T", uplo: str = "U",
 def dstfttr(arf: torch.Tensor, *, transr: str = "T", uplo: str = "U",
             n: int = None) -> torch.Tensor:
     """float64 RFP tensor -> new (n, n) tensor with the uplo triangle filled."""
-    _get_handle, _fill, _, _n_from_rfp, _, _op, _, _ = _pkg()
+    _get_handle, _fill, _, _n_from_rfp, _, _op, _ptr, _ = _pkg()
     _validate64(arf, "arf")
     if n is None:
         n = _n_from_rfp(arf.numel())
-    A = torch.zeros(n, n, dtype=torch.float64, device=arf.device)
-    dstfttr_raw(_get_handle(), _op(transr), _fill(uplo), n, arf, A, n)
+    A = torch.empty(n, n, dtype=torch.float64, device=arf.device)
+    check(_L().curfpDstfttrFill(_get_handle().ptr, _op(transr), _fill(uplo), n, _ptr(arf),
+                                _ptr(A), n))
     return A
 
 

@@ -30,6 +30,8 @@ SIGNATURES = {
     "curfpSstrttf": [_h, _i, _i, _i, _p, _i, _p],
     "curfpSpftri": [_h, _i, _i, _i, _p],
     "curfpSstfttr": [_h, _i, _i, _i, _p, _p, _i],
+    "curfpSstfttrFill": [_h, _i, _i, _i, _p, _p, _i],
+    "curfpDstfttrFill": [_h, _i, _i, _i, _p, _p, _i],
     "curfpSsfr2k": [_h, _i, _i, _i, _i, _i, ctypes.POINTER(_f), _p, _i, _p,
                     _i, ctypes.POINTER(_f), _p],
     "curfpRfpDiagIndices": [_h, _i, _i, _i, _p],

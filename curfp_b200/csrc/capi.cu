@@ -80,7 +80,7 @@ __global__ void diag_zero_check(Geometry g, const T* arf, int* flag) {
 template <typename T>
 curfpStatus_t pack_strided(curfpHandle_t h, int transr, int lower, int n, const T* src,
                            T* dst, int64_t drs, int64_t dcs, int to_rfp,
-                           float diag_scale) {
+                           float diag_scale, int fill = 0) {
   Geometry g = rfp::geometry(n, transr, lower);
   rfp::kpack::PackArgs a{};
   const int tiles = rfp::kpack::pack_blocks(g, &a);
@@ -90,8 +90,8 @@ curfpStatus_t pack_strided(curfpHandle_t h, int transr, int lower, int n, const 
   if (tiles == 0) return CURFP_STATUS_SUCCESS;
   rfp::ProfScope ps(h->prof, h->stream, rfp::K_PACK, 0, (double)sizeof(T) * n * ((double)n + 1));
   rfp::kpack::pack_kernel<T>
-      <<<tiles, dim3(rfp::kpack::TX, rfp::kpack::TY), 0, h->stream>>>(a, src, dst,
-                                                                     to_rfp);
+      <<<tiles, dim3(rfp::kpack::TX, rfp::kpack::TY), 0, h->stream>>>(a, src, dst, to_rfp,
+                                                                     fill);
   ++h->launches;
   return ok_launch() ? CURFP_STATUS_SUCCESS : CURFP_STATUS_EXECUTION_FAILED;
 }
@@ -99,9 +99,9 @@ curfpStatus_t pack_strided(curfpHandle_t h, int transr, int lower, int n, const 
 // strttf / stfttr on a row-major n x n matrix with leading dimension lda.
 template <typename T>
 curfpStatus_t pack(curfpHandle_t h, int transr, int lower, int n, const T* src,
-                   T* dst, int64_t lda, int to_rfp) {
+                   T* dst, int64_t lda, int to_rfp, int fill = 0) {
   return pack_strided(h, transr, lower, n, src, dst, lower ? lda : 1, lower ? 1 : lda,
-                      to_rfp, 1.0f);
+                      to_rfp, 1.0f, fill);
 }
 
 int symm_launch(curfpHandle_t h, const Geometry& g, const float* A, const float* X,
@@ -515,6 +515,25 @@ curfpStatus_t curfpSstfttr(curfpHandle_t handle, curfpOperation_t transr,
   if (n == 0) return CURFP_STATUS_SUCCESS;
   return pack(handle, transr == CURFP_OP_T, uplo == CURFP_FILL_MODE_LOWER, n,
               arf, A, lda, 0);
+}
+
+// Not in the reference's ABI: stfttr into a full square whose other triangle is
+// set to zero (what the Python stfttr returns), in one pass over the square.
+curfpStatus_t curfpSstfttrFill(curfpHandle_t handle, curfpOperation_t transr,
+                               curfpFillMode_t uplo, int n, const float* arf, float* A, int lda) {
+  if (!handle) return CURFP_STATUS_NOT_INITIALIZED;
+  if (n < 0 || lda < n) return CURFP_STATUS_INVALID_VALUE;
+  if (n == 0) return CURFP_STATUS_SUCCESS;
+  return pack(handle, transr == CURFP_OP_T, uplo == CURFP_FILL_MODE_LOWER, n, arf, A, lda, 0, 1);
+}
+
+curfpStatus_t curfpDstfttrFill(curfpHandle_t handle, curfpOperation_t transr,
+                               curfpFillMode_t uplo, int n, const double* arf, double* A,
+                               int lda) {
+  if (!handle) return CURFP_STATUS_NOT_INITIALIZED;
+  if (n < 0 || lda < n) return CURFP_STATUS_INVALID_VALUE;
+  if (n == 0) return CURFP_STATUS_SUCCESS;
+  return pack(handle, transr == CURFP_OP_T, uplo == CURFP_FILL_MODE_LOWER, n, arf, A, lda, 0, 1);
 }
 
 // curfp/__init__.py:194-269

@@ -149,6 +149,14 @@ curfpStatus_t curfpSstfttr(curfpHandle_t handle, curfpOperation_t transr,
                            curfpFillMode_t uplo, int n, const float *arf,
                            float *A, int lda);
 
+/* The same into a full square: the other triangle is set to zero. */
+curfpStatus_t curfpSstfttrFill(curfpHandle_t handle, curfpOperation_t transr,
+                               curfpFillMode_t uplo, int n, const float *arf,
+                               float *A, int lda);
+curfpStatus_t curfpDstfttrFill(curfpHandle_t handle, curfpOperation_t transr,
+                               curfpFillMode_t uplo, int n, const double *arf,
+                               double *A, int lda);
+
 /* C := alpha*(op(A)op(B)^T + op(B)op(A)^T) + beta*C in RFP.
  * Replaces include/curfp.h:305-319 (src/curfp_ssfr2k.cpp:121-232). */
 curfpStatus_t curfpSsfr2k(curfpHandle_t handle, curfpOperation_t transr,
