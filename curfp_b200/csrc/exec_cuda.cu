@@ -7,6 +7,7 @@
 
 #include "context.h"
 #include "k_chain.cuh"
+#include "k_chain1.cuh"
 #include "k_chol.cuh"
 #include "k_gemm.cuh"
 #include "gemm_route.h"
@@ -634,6 +635,32 @@ int launch_chain(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int n, Vi
   ++ctx->wait_launches;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
+// One FP32 right-hand side (k_chain1.cuh).
+int launch_chain1(curfpContext* ctx, const int* abort_flag, View L, int n, View B, float alpha,
+                  const float* W) {
+  kchain1::Args a{};
+  a.L = L; a.B = B;
+  a.n = n;
+  a.nblk = (n + kchain::NB - 1) / kchain::NB;
+  a.alpha = alpha;
+  a.W = W;
+  const size_t words = (size_t)a.nblk * kchain::NB + 1;  // the ticket follows the words
+  a.ws = static_cast<unsigned long long*>(
+      grow_buffer(ctx, &ctx->tsv, &ctx->tsv_bytes, words * sizeof(unsigned long long)));
+  if (!a.ws) return 2;
+  if (cudaMemsetAsync(a.ws, 0, words * sizeof(unsigned long long), ctx->stream) != cudaSuccess)
+    return 4;
+  a.sync = reinterpret_cast<int*>(a.ws + words - 1);
+  a.err = ctx->d_info + 1;
+  a.abort_flag = abort_flag;
+  ProfScope ps(ctx->prof, ctx->stream, K_TRSV, (double)n * n, (double)n * n * 2.0);
+  ps.shape(n, 1, n, a.nblk);
+  kchain1::chain1<<<(a.nblk + kchain::CS - 1) / kchain::CS * kchain::CS, kchain1::THR, 0,
+                    ctx->stream>>>(a);
+  ++ctx->launches;
+  ++ctx->wait_launches;
+  return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
 }  // namespace
 
 // Up to kTrsvMaxRhs right-hand sides (FP64 128): the chain inside clusters, in
@@ -641,7 +668,7 @@ int launch_chain(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int n, Vi
 // with the chunk while the products' cost per column grows: 8 columns up to
 // 256 (block row, chunk) pairs, 16 up to 512, else 32 (8192 rows, 16 / 64 / 128
 // columns: 8 wide 190 / 510 / 970 us, 16 wide 262 / 390 / 690 us, 32 wide 400 /
-// 420 / 600 us; FP64 8 wide).  More right-hand sides keep every SM busy:
+// 420 / 600 us; FP64 8 wide); a single FP32 column has its own kernel.  More right-hand sides keep every SM busy:
 // 64-column chunks handed on through L2 (n = 512 leaves of the recursion).
 template <typename T>
 int CudaExecT<T>::trsm_wave(ViewT<T> L, int n, ViewT<T> B, int m, T alpha, const T* W) {
@@ -649,6 +676,7 @@ int CudaExecT<T>::trsm_wave(ViewT<T> L, int n, ViewT<T> B, int m, T alpha, const
   const int nblk = (n + kTrsmLeaf - 1) / kTrsmLeaf;
   if (m <= (sizeof(T) == 4 ? kTrsvMaxRhs : 128)) {
     if constexpr (sizeof(T) == 4) {
+      if (m == 1) return launch_chain1(ctx_, abort_, L, n, B, alpha, W);
       if ((int64_t)nblk * ((m + 15) / 16) > 512)
         return launch_chain<T, 32>(ctx_, abort_, L, n, B, m, alpha, W);
       if ((int64_t)nblk * ((m + 7) / 8) > 256)
