@@ -35,16 +35,19 @@
 // (n2 x n1) and V22 (n2 x n2) of an RFP array.  The first nbf tile columns
 // are factored: all of them, or only the first block's (then V21 becomes
 // V21 L11^-T and V22 is not touched; a plain matrix has n2 = 0).
-// Bound by the chain: a 64-column step takes 13.5 us in FP32 and 23.6 us in
-// FP64 (n = 2000; about 5 us of it the two 32-column factors), against ~50 us
-// per 64 columns of the recursion with 128-row tiles.  RFP factorizations on
-// B200, recursion -> this: n = 250 0.19 -> 0.060 ms, n = 4095 4.3 -> 1.14 ms
-// (with one tensor-core update), FP64 n = 3000 4.8 -> 1.2 ms.
+// Bound by the chain: a 64-column step takes 12.9 us in FP32 and 24.7 us in
+// FP64 (n = 2000; 5.8 us of it the two 32-column factors, 180 cycles a column:
+// one warp's instruction issue, which paired FMAs relieve and pairs of columns
+// with their extra products do not), against ~50 us per 64 columns of the
+// recursion with 128-row tiles.  RFP factorizations on B200, recursion -> this:
+// n = 250 0.19 -> 0.055 ms, n = 4095 4.3 -> 1.02 ms (with one tensor-core
+// update), FP64 n = 3000 4.8 -> 1.3 ms.
 // Waits are bounded; a CTA that gives up (or whose diagonal tile has a
 // non-positive pivot) publishes poisoned flags so that its dependents stop.
 #pragma once
 #include <climits>
 #include <cstdint>
+#include <type_traits>
 
 #include "engine.h"
 #include "k_micro.cuh"
@@ -120,15 +123,35 @@ __device__ __forceinline__ double rsqrt_newton(double d) {
   return fma(0.5 * r, fma(-d * r, r, 1.0), r);
 }
 
+// x_k += f l_k for K0 <= k < 32, two at a time in FP32 (one warp issues these
+// alone, so their number is what counts).
+template <int K0, typename T>
+__device__ __forceinline__ void axpy(T (&x)[32], T f, const T (&l)[32]) {
+  if constexpr (sizeof(T) == 4) {
+    if constexpr (K0 < 32 && K0 % 2 == 1) x[K0] = fma(f, l[K0], x[K0]);
+#pragma unroll
+    for (int k = (K0 + 1) & ~1; k < 32; k += 2) fma2(x[k], x[k + 1], l[k], l[k + 1], f, f);
+  } else {
+#pragma unroll
+    for (int k = K0; k < 32; ++k) x[k] = fma(f, l[k], x[k]);
+  }
+}
+// The compile-time index of an unrolled loop.
+template <int J, typename F>
+__device__ __forceinline__ void each_column(F f) {
+  if constexpr (J < 32) {
+    f(std::integral_constant<int, J>{});
+    each_column<J + 1>(f);
+  }
+}
+
 // One warp, lane = row: Cholesky factor of a 32 x 32 block s (column-major,
 // stride 64; lower triangle read, overwritten by the factor; garbage above
 // the diagonal).  The chain of a column is: update the next column, its pivot
 // by shuffle, rsqrt, scale.  The column goes to raw (32 x 32, column-major)
 // unscaled: it comes back as 16-byte broadcast reads behind the rsqrt, and
 // drives the inverse in another warp, which is let on every 8 columns
-// (barriers bar0 .. bar0 + 3).  After a failed pivot the remaining columns of
-// raw are not written, but all barriers are passed.  Returns 0, or 1 + the
-// failing column.
+// (barriers bar0 .. bar0 + 3).  Returns 0, or 1 + the failing column.
 template <typename T>
 __device__ __forceinline__ int factor32(T* s, T* raw, int bar0) {
   const int lane = threadIdx.x & 31;
@@ -139,29 +162,29 @@ __device__ __forceinline__ int factor32(T* s, T* raw, int bar0) {
   raw[lane] = a[0];
   T d = __shfl_sync(0xffffffffu, a[0], 0);
   __syncwarp();
+  each_column<0>([&](auto jc) {
+    constexpr int j = decltype(jc)::value;
+    // No branch on the pivot: straight-line code lets a column's updates fill
+    // the next one's chain.  From a failed pivot on, r = 0 leaves everything
+    // as it is.
+    fail = fail == 0 && !(d > T(0)) ? j + 1 : fail;  // the same value in every lane
+    const T r = fail ? T(0) : rsqrt_newton(d);
+    T lk[32];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    if (!fail && !(d > T(0))) fail = j + 1;  // the same value in every lane
-    if (!fail) {
-      const T r = rsqrt_newton(d);
-      T lk[32];
-#pragma unroll
-      for (int v4 = (j + 1) / 4; v4 < 8; ++v4)
-        lds4(raw + j * 32 + 4 * v4, *reinterpret_cast<T(*)[4]>(lk + 4 * v4));
-      const T l = a[j] * r, t = l * r, dj = d;
-      if (j + 1 < 32) {
-        a[j + 1] = fma(-t, lk[j + 1], a[j + 1]);
-        d = __shfl_sync(0xffffffffu, a[j + 1], j + 1);
-        raw[(j + 1) * 32 + lane] = a[j + 1];
-        __syncwarp();
-      }
-      // the diagonal element: sqrt(d) = d r corrected by its residual
-      a[j] = lane == j ? fma(T(0.5) * r, fma(-l, l, dj), l) : l;
-#pragma unroll
-      for (int k = j + 2; k < 32; ++k) a[k] = fma(-t, lk[k], a[k]);
+    for (int v4 = (j + 1) / 4; v4 < 8; ++v4)
+      lds4(raw + j * 32 + 4 * v4, *reinterpret_cast<T(*)[4]>(lk + 4 * v4));
+    const T l = a[j] * r, t = l * r, dj = d;
+    if constexpr (j + 1 < 32) {
+      a[j + 1] = fma(-t, lk[j + 1], a[j + 1]);
+      d = __shfl_sync(0xffffffffu, a[j + 1], j + 1);
+      raw[(j + 1) * 32 + lane] = a[j + 1];
+      __syncwarp();
     }
+    // the diagonal element: sqrt(d) = d r corrected by its residual
+    a[j] = fail ? a[j] : (lane == j ? fma(T(0.5) * r, fma(-l, l, dj), l) : l);
+    axpy<j + 2>(a, -t, lk);
     if ((j & 7) == 7) bar_arrive_id<64>(bar0 + (j >> 3));
-  }
+  });
 #pragma unroll
   for (int k = 0; k < 32; ++k) s[k * NB + lane] = a[k];
   return fail;
@@ -176,8 +199,8 @@ __device__ __forceinline__ void inverse32(T* w, const T* raw, int bar0) {
   T x[32];
 #pragma unroll
   for (int k = 0; k < 32; ++k) x[k] = k == lane ? T(1) : T(0);
-#pragma unroll
-  for (int j = 0; j < 32; ++j) {
+  each_column<0>([&](auto jc) {
+    constexpr int j = decltype(jc)::value;
     if ((j & 7) == 0) bar_sync_id<64>(bar0 + (j >> 3));
     T lk[32];
 #pragma unroll
@@ -186,9 +209,8 @@ __device__ __forceinline__ void inverse32(T* w, const T* raw, int bar0) {
     const T r = rsqrt_newton(lk[j]);
     const T u = x[j] * r, v = u * r;
     x[j] = u;
-#pragma unroll
-    for (int k = j + 1; k < 32; ++k) x[k] = fma(-v, lk[k], x[k]);
-  }
+    axpy<j + 1>(x, -v, lk);
+  });
 #pragma unroll
   for (int k = 0; k < 32; k += 4) {
     const T v[4] = {x[k], x[k + 1], x[k + 2], x[k + 3]};
@@ -462,8 +484,11 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
 
   // Diagonal tile by 32 x 32 quarters: D0 and its inverse by warps 0 and 1,
   // while the last quarter of the warps on the SMSPs that hold neither form
-  // X's lower rows and the rest of S.
+  // X's lower rows and S10 (FP64 S11 too).
   constexpr int SH = THR / 2;  // threads of the shadow work: warps w with w % 4 >= 2
+  // In FP32 the shadow work is the longer side, so S11's product with X goes
+  // beside L10; in FP64 the factor is (n = 2000: 755 against 800 us).
+  constexpr bool kBeside = sizeof(T) == 4;
   const bool shadow = (warp & 3) >= 2;
   const int st = ((warp >> 2) * 2 + (warp & 1)) * 32 + lane;
 #pragma unroll 1
@@ -487,13 +512,18 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
           }
         }
         bar_sync<10, SH>();
-        {
+        if constexpr (kBeside) {
+          // S10 -= X1 X0^T (S11's share follows beside L10)
+          constexpr int SG = SH / 64, KS = NB / SG;
+          const int sg = st >> 6, v = st & 63, tr = v & 7, tc = v >> 3;
+          product4<NB, NB>(o, Xs + 32, Xs, sg * KS, sg * KS + KS, tr, tc);
+          reduce4<SG, 64, 10>(o, red, sg, v);
+          if (sg == 0) put4<NB, true>(Ss + 32, o, tr, tc);
+        } else {
           // S10 -= X1 X0^T and S11 -= X1 X1^T, 64 threads each
-          constexpr int SG = SH / 128, KS = NB / SG;
-          const int sg = st >> 7, v = st & 127, w = v & 63, q11 = v >> 6, tr = w & 7, tc = w >> 3;
-          product4<NB, NB>(o, Xs + 32, Xs + 32 * q11, sg * KS, sg * KS + KS, tr, tc);
-          reduce4<SG, 128, 10>(o, red, sg, v);
-          if (sg == 0) put4<NB, true>(Ss + 32 * q11 * NB + 32, o, tr, tc);
+          const int v = st & 63, q11 = st >> 6, tr = v & 7, tc = v >> 3;
+          product4<NB, NB>(o, Xs + 32, Xs + 32 * q11, 0, NB, tr, tc);
+          put4<NB, true>(Ss + 32 * q11 * NB + 32, o, tr, tc);
         }
         if (st == SH - 1) ktrsv::st_release(&flags[tidx(i, c)], 1);  // X, ordered by the barriers
       }
@@ -515,16 +545,25 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
     }
     __syncthreads();
     if (sh_fail || h == 1) break;
-    // L10 = S10 inv(D0)^T, then S11 -= L10 L10^T: 4 x 4 on two groups of 64
+    // Half of the groups: L10 = S10 inv(D0)^T; with kBeside the others
+    // S11 -= X1 X1^T.  Then S11 -= L10 L10^T.
     T o[4][4];
     const int tr = u & 7, tc = u >> 3;
-    if (grp < 2) {
-      product4<NB, LDW>(o, Ss + 32, Ws, grp * 16, min(grp * 16 + 16, tc * 4 + 4), tr, tc);
-      reduce4<2, 64, 1>(o, red, grp, u);
+    constexpr int HG = G / 2, KL = 32 / HG, KX = NB / HG;
+    if (grp < HG) {
+      product4<NB, LDW>(o, Ss + 32, Ws, grp * KL, min(grp * KL + KL, tc * 4 + 4), tr, tc);
+      reduce4<HG, 64, 1>(o, red, grp, u);
       if (grp == 0) put4<32, false>(Lb, o, tr, tc);
-      bar_sync<1, 128>();
-      product4<32, 32>(o, Lb, Lb, grp * 16, grp * 16 + 16, tr, tc);
-      reduce4<2, 64, 1>(o, red + 1024, grp, u);
+    } else if (kBeside && c >= 0) {
+      const int xg = grp - HG;
+      product4<NB, NB>(o, Xs + 32, Xs + 32, xg * KX, xg * KX + KX, tr, tc);
+      reduce4<HG, 64, 11>(o, Wc, xg, u);  // W_c has served
+      if (xg == 0) put4<NB, true>(Ss + 32 * NB + 32, o, tr, tc);
+    }
+    __syncthreads();
+    if (grp < HG) {
+      product4<32, 32>(o, Lb, Lb, grp * KL, grp * KL + KL, tr, tc);
+      reduce4<HG, 64, 1>(o, red, grp, u);
       if (grp == 0) put4<NB, true>(Ss + 32 * NB + 32, o, tr, tc);
     }
     __syncthreads();
