@@ -75,22 +75,35 @@ int stage(curfpContext* ctx, void** buf, size_t* cur, View X, int rows, int k, i
   unsigned* maxbits = reinterpret_cast<unsigned*>(out->scale + out->rows_pad);
   ProfScope ps(ctx->prof, ctx->stream, K_TC_STAGE, 0,
                (double)rows * k * 8.0 + (double)out->rows_pad * out->k_pad * 2.0 * planes);
-  const int groups = out->rows_pad / 32;
+  // Wide reads need a unit stride forward, every vector 16-byte aligned, and
+  // no mask (masked elements are not to be read).
+  const int64_t other = X.cs == 1 ? X.rs : X.cs;
+  const bool wide = mask == 0 && (X.cs == 1 || X.rs == 1) && other % 4 == 0 &&
+                    (reinterpret_cast<uintptr_t>(X.p) & 15) == 0;
+  const bool kc = X.cs == 1;
+  const int groups = out->rows_pad / (wide && !kc ? 128 : 32);
   const int kchunks = k > 0 ? (k + 127) / 128 : 1;
   int nsplit = (8 * sm_count(ctx) + groups - 1) / groups;
   if (nsplit > kchunks) nsplit = kchunks;
   const int kseg = 128 * ((kchunks + nsplit - 1) / nsplit);
   const int ksplit = k > 0 ? (k + kseg - 1) / kseg : 1;
-  if (ksplit > 1 &&
-      cudaMemsetAsync(maxbits, 0, (size_t)out->rows_pad * sizeof(unsigned), ctx->stream) !=
-          cudaSuccess)
+  const int atomic = ksplit > 1 ? 1 : 0;
+  if (atomic && cudaMemsetAsync(maxbits, 0, (size_t)out->rows_pad * sizeof(unsigned),
+                                ctx->stream) != cudaSuccess)
     return 4;
-  ktc::rowmax_kernel<<<dim3(groups, ksplit), 256, 0, ctx->stream>>>(
-      X, rows, k, kseg, maxbits, mask, koff, ksplit > 1 ? 1 : 0);
-  dim3 grid(out->k_pad / 64, out->rows_pad / 32);
-  ktc::digits_kernel<<<grid, dim3(32, 8), 0, ctx->stream>>>(X, rows, k, maxbits, out->scale,
-                                                            out->p, out->rows_pad, out->k_pad,
-                                                            planes, mask, koff);
+  const dim3 mgrid(groups, ksplit), dgrid(out->k_pad / 64, out->rows_pad / 64);
+  if (!wide)
+    ktc::rowmax_kernel<<<mgrid, 256, 0, ctx->stream>>>(X, rows, k, kseg, maxbits, mask, koff,
+                                                       atomic);
+  else if (kc)
+    ktc::rowmax_wide<true><<<mgrid, 256, 0, ctx->stream>>>(X, rows, k, kseg, maxbits, atomic);
+  else
+    ktc::rowmax_wide<false><<<mgrid, 256, 0, ctx->stream>>>(X, rows, k, kseg, maxbits, atomic);
+  const auto digits = !wide ? ktc::digits_kernel<ktc::READ_ANY>
+                      : kc  ? ktc::digits_kernel<ktc::READ_K>
+                            : ktc::digits_kernel<ktc::READ_ROWS>;
+  digits<<<dgrid, 256, 0, ctx->stream>>>(X, rows, k, maxbits, out->scale, out->p, out->rows_pad,
+                                         out->k_pad, planes, mask, koff);
   ctx->launches += 2;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
