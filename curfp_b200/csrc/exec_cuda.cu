@@ -663,13 +663,55 @@ int launch_chain1(curfpContext* ctx, const int* abort_flag, View L, int n, View 
 }
 }  // namespace
 
+namespace {
+// Many right-hand sides: 64 x 64 tiles handed on through the workspace (k_tri.cuh).
+template <typename T>
+int launch_solve_tiles(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int n, ViewT<T> B,
+                       int m, T alpha, const T* W) {
+  ktri::SolveArgs<T> a{};
+  a.B = B;
+  a.n = n; a.m = m;
+  a.nblk = (n + ktri::NB - 1) / ktri::NB;
+  a.nchunk = (m + ktri::NB - 1) / ktri::NB;
+  a.alpha = alpha;
+  a.W = W;
+  const size_t tiles = (size_t)a.nblk * a.nchunk, words = 1 + tiles;
+  const int lower = a.nblk * (a.nblk - 1) / 2;  // packed tiles of L, then X's
+  T* const ws = static_cast<T*>(grow_buffer(
+      ctx, &ctx->wst, &ctx->wst_bytes,
+      (lower + tiles - a.nchunk + 1) * ktri::TILE * sizeof(T)));
+  a.Lp = ws;
+  a.ws = ws + (size_t)lower * ktri::TILE;
+  a.sync = static_cast<int*>(grow_buffer(ctx, &ctx->tsv, &ctx->tsv_bytes, words * sizeof(int)));
+  if (!ws || !a.sync) return 2;
+  if (cudaMemsetAsync(a.sync, 0, words * sizeof(int), ctx->stream) != cudaSuccess) return 4;
+  a.err = ctx->d_info + 1;
+  a.abort_flag = abort_flag;
+  constexpr int smem = ktri::smem_bytes<T>();
+  static const bool attr = smem_attr(ktri::solve_tiles<T>, smem);
+  if (!attr) return 4;
+  ProfScope ps(ctx->prof, ctx->stream, K_TRSV, (double)n * n * m, (double)n * n * sizeof(T) / 2.0);
+  ps.shape(n, m, n, (int)tiles);
+  if (lower > 0) {
+    ktri::pack_lower<T><<<lower, ktri::THR, 0, ctx->stream>>>(L, n, ws, abort_flag);
+    ++ctx->launches;
+  }
+  ktri::solve_tiles<T><<<(int)tiles, ktri::THR, smem, ctx->stream>>>(a);
+  ++ctx->launches;
+  ++ctx->wait_launches;
+  return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+}  // namespace
+
 // Up to kTrsvMaxRhs right-hand sides (FP64 128): the chain inside clusters, in
 // chunks as narrow as the throughput allows, since the chain's step shrinks
 // with the chunk while the products' cost per column grows: 8 columns up to
 // 256 (block row, chunk) pairs, 16 up to 512, else 32 (8192 rows, 16 / 64 / 128
 // columns: 8 wide 190 / 510 / 970 us, 16 wide 262 / 390 / 690 us, 32 wide 400 /
-// 420 / 600 us; FP64 8 wide); a single FP32 column has its own kernel.  More right-hand sides keep every SM busy:
-// 64-column chunks handed on through L2 (n = 512 leaves of the recursion).
+// 420 / 600 us; FP64 8 wide); a single FP32 column has its own kernel.  More right-hand sides keep every SM busy
+// (n = 512 leaves of the recursion): 64-column chunks handed on through L2, in
+// FP32 from kSolveTilesRhs columns on by the kernel made for throughput (512
+// rows, 2048 / 4096 / 16384 columns: 70 / 88 / 208 us, there 77 / 79 / 148).
 template <typename T>
 int CudaExecT<T>::trsm_wave(ViewT<T> L, int n, ViewT<T> B, int m, T alpha, const T* W) {
   if (n <= 0 || m <= 0) return 0;
@@ -684,6 +726,8 @@ int CudaExecT<T>::trsm_wave(ViewT<T> L, int n, ViewT<T> B, int m, T alpha, const
     }
     return launch_chain<T, 8>(ctx_, abort_, L, n, B, m, alpha, W);
   }
+  if constexpr (sizeof(T) == 4)
+    if (m >= kSolveTilesRhs) return launch_solve_tiles<T>(ctx_, abort_, L, n, B, m, alpha, W);
   return launch_wave<T, 64>(ctx_, abort_, L, n, B, m, alpha, W);
 }
 

@@ -1,4 +1,5 @@
-// k_tri.cuh — inverse of a lower triangular block by a wave of 64 x 64 tiles.
+// k_tri.cuh — inverse of a lower triangular block, and solves with many
+// right-hand sides (solve_tiles), by waves of 64 x 64 tiles.
 //
 // M = L^-1 in one launch (and one that stores it): tickets in row order, so a
 // CTA waits only on smaller tickets and no co-residency is needed.  CTA (i, c),
@@ -190,6 +191,184 @@ __global__ void __launch_bounds__(THR, sizeof(T) == 4 ? 2 : 1) inverse_wave(cons
   }
   __syncthreads();
   if (tid == 0) ktrsv::st_release(flag(i), 1);
+}
+
+// L X = alpha B (B n x m view, X over B) by a wave of 64 x 64 tiles: CTA (i, c),
+// tickets in row order,
+//   X_ic = W_i (alpha B_ic - sum_{k<i} L_ik X_kc),
+// for the many right-hand sides of the recursion's leaves, where throughput
+// counts and not the chain: 8 x 8 register products, two CTAs per SM, L packed
+// beforehand (pack_lower) and X published in the workspace so that both are
+// fetched 16 bytes at a time.  Bound by the products' shared-memory reads and
+// FMA issue.  512 rows and 16384 / 8192 / 4096 columns take 148 / 91 / 79 us
+// with the packing; with 4-byte copies of L from the matrix 172 / 100 / 81 us;
+// ktrsv::trsm_wave (4 x 4 register products) 208 / 118 / 88 us.
+template <typename T>
+struct SolveArgs {
+  ViewT<T> B;
+  const T* Lp;  // pack_lower's tiles
+  int n, m, nblk, nchunk;
+  T alpha;
+  const T* W;
+  T* ws;
+  int* sync;  // [0] ticket, [1 + i * nchunk + c] flags
+  int* err;
+  const int* abort_flag;
+};
+
+// The tiles (i, k), k < i, of L, k-major, at tile_at(i - 1, k) of ws.
+template <typename T>
+__global__ void __launch_bounds__(THR) pack_lower(ViewT<T> L, int n, T* ws,
+                                                  const int* abort_flag) {
+  if (abort_flag && *abort_flag != INT_MAX) return;
+  __shared__ T s[NB * (NB + 1)];
+  int i, k;
+  tile_of((int)blockIdx.x, i, k);
+  const int rows = min(NB, n - (i + 1) * NB);
+  ktrsv::load_tile<NB + 1>(s, sub(L, (int64_t)(i + 1) * NB, (int64_t)k * NB), rows, NB);
+  ktrsv::cp_commit();
+  ktrsv::cp_wait_all();
+  __syncthreads();
+#pragma unroll 4
+  for (int q = 0; q < TILE / THR; ++q) {
+    const int e = threadIdx.x + THR * q;
+    ws[(int64_t)blockIdx.x * TILE + e] = s[(e / NB) * (NB + 1) + e % NB];
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(THR, sizeof(T) == 4 ? 2 : 1) solve_tiles(const SolveArgs<T> g) {
+  if (g.abort_flag && *g.abort_flag != INT_MAX) return;
+  extern __shared__ __align__(16) unsigned char tri_raw[];
+  T* Ls = reinterpret_cast<T*>(tri_raw);
+  T* Xs = Ls + 2 * NB * LDL;
+  T* Ws = Xs + 2 * TILE;
+  T* Ts = Ws + TILE;
+  __shared__ int sh_ticket, sh_state[2];  // tile k's state at k & 1
+  const int tid = threadIdx.x, grp = tid >> 6, u = tid & 63;
+  if (tid == 0) sh_ticket = atomicAdd(g.sync, 1);
+  __syncthreads();
+  const int i = sh_ticket / g.nchunk, c = sh_ticket % g.nchunk;
+  const int rows = min(NB, g.n - i * NB), cols = min(NB, g.m - c * NB);
+  int* const flags = g.sync + 1 + c;  // tile (k, c) at k * nchunk
+  T* const xs = g.ws + (int64_t)c * TILE;
+  constexpr int VW = 16 / (int)sizeof(T);
+
+  auto load_l = [&](int k) {
+    T* s = Ls + (k & 1) * NB * LDL;
+    const T* l = g.Lp + (int64_t)tile_at(i - 1, k) * TILE;
+#pragma unroll
+    for (int w = 0; w < TILE / VW / THR; ++w) {
+      const int e = (tid + THR * w) * VW;
+      cp16(s + (e / NB) * LDL + e % NB, l + e);
+    }
+  };
+  auto load_x = [&](int k) {
+    T* s = Xs + (k & 1) * TILE;
+    const T* x = xs + (int64_t)k * g.nchunk * TILE;
+#pragma unroll
+    for (int w = 0; w < TILE / VW / THR; ++w) {
+      const int e = (tid + THR * w) * VW;
+      cp16(s + e, x + e);
+    }
+  };
+  // Thread 0 waits for tile k; the block barrier that follows tells the rest.
+  auto wait = [&](int k) {
+    if (tid == 0) sh_state[k & 1] = ktrsv::wait_flag(&flags[(int64_t)k * g.nchunk], g.err);
+  };
+
+  if (i > 0) load_l(0);
+  {
+    const T* w = g.W + (int64_t)i * kInvStride;
+#pragma unroll
+    for (int q = 0; q < TILE / VW / THR; ++q) {
+      const int e = (tid + THR * q) * VW;
+      cp16(Ws + e, w + e);
+    }
+  }
+  // T = alpha B_ic, read along B's contiguous index
+  const ViewT<T> Bv = sub(g.B, (int64_t)i * NB, (int64_t)c * NB);
+  const bool rowcont = (Bv.cs == 1 || Bv.cs == -1) && !(Bv.rs == 1 || Bv.rs == -1);
+#pragma unroll 8
+  for (int q = 0; q < TILE / THR; ++q) {
+    const int e = tid + THR * q, a = rowcont ? e / NB : e % NB, b = rowcont ? e % NB : e / NB;
+    Ts[a * LDL + b] = a < rows && b < cols ? g.alpha * Bv.p[a * Bv.rs + b * Bv.cs] : T(0);
+  }
+  if (i > 0) {
+    wait(0);
+    __syncthreads();
+    bool good = sh_state[0] >= 0;
+    if (good) load_x(0);
+    ktrsv::cp_commit();
+    T acc[8][8];
+#pragma unroll
+    for (int p = 0; p < 8; ++p)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[p][q] = T(0);
+    for (int k = 0; good && k < i; ++k) {
+      const bool more = k + 1 < i;
+      ktrsv::cp_wait_all();
+      if (more) wait(k + 1);
+      __syncthreads();  // tile k landed; every thread is done with the other buffers
+      if (more) {
+        good = sh_state[(k + 1) & 1] >= 0;
+        load_l(k + 1);
+        if (good) load_x(k + 1);
+        ktrsv::cp_commit();
+      }
+      // rows of the register tile: X's columns, columns: L's rows
+      product8<NB, LDL, NB / G>(acc, Xs + (k & 1) * TILE, Ls + (k & 1) * NB * LDL,
+                                grp * (NB / G), u);
+    }
+    if (!good) {  // the same in every thread
+      ktrsv::cp_wait_all();
+      __syncthreads();
+      if (tid == 0) ktrsv::st_release(&flags[(int64_t)i * g.nchunk], -1);
+      return;
+    }
+    // T -= the groups' partial sums, which meet in the operand buffers
+    __syncthreads();
+    store8(Ls + grp * TILE, acc, u);
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < TILE / 4 / THR; ++w) {
+      const int e = (tid + THR * w) * 4;
+      T* t = Ts + (e / NB) * LDL + e % NB;
+      T s[4], v[4];
+      lds4(Ls + e, s);
+#pragma unroll
+      for (int q = 1; q < G; ++q) {
+        lds4(Ls + q * TILE + e, v);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) s[r] += v[r];
+      }
+      lds4(t, v);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) v[r] -= s[r];
+      sts4(t, v);
+    }
+  }
+  ktrsv::cp_commit();
+  ktrsv::cp_wait_all();
+  __syncthreads();
+  // X = W_i T: W_i(a, k) = 0 for k > a
+  T o[4][4];
+  const int tr = tid & 15, tc = tid >> 4;
+  product4<LDL, NB>(o, Ts, Ws, 0, tc * 4 + 4, tr, tc);
+  if (i + 1 < g.nblk) {
+    put4<NB, false>(xs + (int64_t)i * g.nchunk * TILE, o, tr, tc);
+    __syncthreads();
+    if (tid == 0) ktrsv::st_release(&flags[(int64_t)i * g.nchunk], 1);
+  } else {
+    __syncthreads();
+  }
+  put4<LDL, false>(Ts, o, tr, tc);
+  __syncthreads();
+#pragma unroll 8
+  for (int q = 0; q < TILE / THR; ++q) {
+    const int e = tid + THR * q, a = rowcont ? e / NB : e % NB, b = rowcont ? e % NB : e / NB;
+    if (a < rows && b < cols) Bv.p[a * Bv.rs + b * Bv.cs] = Ts[a * LDL + b];
+  }
 }
 
 // The inverse's published tiles -> the lower triangle of L.
