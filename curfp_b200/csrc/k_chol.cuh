@@ -487,7 +487,8 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
   // X's lower rows and S10 (FP64 S11 too).
   constexpr int SH = THR / 2;  // threads of the shadow work: warps w with w % 4 >= 2
   // In FP32 the shadow work is the longer side, so S11's product with X goes
-  // beside L10; in FP64 the factor is (n = 2000: 755 against 800 us).
+  // beside L10 (n = 2000: 414 against 440 us); in FP64 the factor is longer and
+  // both ways take the same time, so its order stays.
   constexpr bool kBeside = sizeof(T) == 4;
   const bool shadow = (warp & 3) >= 2;
   const int st = ((warp >> 2) * 2 + (warp & 1)) * 32 + lane;
