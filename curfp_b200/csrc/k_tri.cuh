@@ -199,8 +199,8 @@ __global__ void __launch_bounds__(THR, sizeof(T) == 4 ? 2 : 1) inverse_wave(cons
 // for the many right-hand sides of the recursion's leaves, where throughput
 // counts and not the chain: 8 x 8 register products, two CTAs per SM, L packed
 // beforehand (pack_lower) and X published in the workspace so that both are
-// fetched 16 bytes at a time.  Bound by the products' shared-memory reads and
-// FMA issue.  512 rows and 16384 / 8192 / 4096 columns take 148 / 91 / 79 us
+// fetched 16 bytes at a time.  The products' shared-memory reads take half
+// of the time, the CTAs' starts, reductions and stores the rest.  512 rows and 16384 / 8192 / 4096 columns take 148 / 91 / 79 us
 // with the packing; with 4-byte copies of L from the matrix 172 / 100 / 81 us;
 // ktrsv::trsm_wave (4 x 4 register products) 208 / 118 / 88 us.
 template <typename T>
