@@ -91,10 +91,9 @@ int launch_gemm(const GemmProbT<T>* p, int count, const int* abort_flag,
   int splits = 1;
   const kgemm::Prob<T>& q0 = b.p[0];
   if (alloc && cnt == 1 && !q0.k2 && !q0.a_tri && !q0.b_tri && !q0.c_lower && !p[0].inplace) {
-    splits = std::min(2 * 148 / tiles, q0.k / 128);
-    if (splits < 2) splits = 1;
-    b.kseg = ((q0.k + splits - 1) / splits + 31) / 32 * 32;
-    splits = (q0.k + b.kseg - 1) / b.kseg;
+    const KSplit ks = tile_split(tiles, q0.k);
+    splits = ks.splits;
+    b.kseg = ks.kseg;
   }
   if (splits > 1) {
     b.part = static_cast<T*>(grow_buffer(ctx, &ctx->wst, &ctx->wst_bytes,
@@ -123,12 +122,11 @@ int launch_skinny(const GemmProbT<T>& g0, const int* abort_flag, curfpContext* c
                      g.m, g.n, g.k, g.alpha, g.beta, g.k, nullptr};
   ProfScope ps(ctx->prof, ctx->stream, K_SGEMM, 2.0 * g.m * g.n * (double)g.k,
                (double)sizeof(T) * g.m * (double)g.k);
-  // about eight CTAs per SM, at least 512 columns each
   int splits = 1;
   if (alloc) {
-    splits = (int)std::min<int64_t>((int64_t)8 * 148 * 32 / g.m + 1, (g.k + 511) / 512);
-    a.kseg = ((g.k + splits - 1) / splits + 31) / 32 * 32;
-    splits = (g.k + a.kseg - 1) / a.kseg;
+    const KSplit ks = skinny_split(g.m, g.k);
+    splits = ks.splits;
+    a.kseg = ks.kseg;
   }
   if (splits > 1) {
     a.part = static_cast<T*>(grow_buffer(ctx, &ctx->wst, &ctx->wst_bytes,

@@ -1,6 +1,9 @@
 // gemm_route.h — which contractions the few-column kernels (k_skinny.cuh)
-// take; host code, shared by the CUDA executor and the host tests.
+// take and how k is split over CTAs; host code, shared by the CUDA executor
+// and the host tests.
 #pragma once
+#include <algorithm>
+
 #include "engine.h"
 
 namespace rfp {
@@ -41,6 +44,27 @@ inline SkinnyRoute skinny_route(const GemmProbT<T>& g0, GemmProbT<T>* out) {
   r.inst = g.n == 1 ? 1 : (g.n == 2 ? 2 : (g.n <= 4 ? 4 : 8));
   *out = g;
   return r;
+}
+
+// k cut into `splits` ranges of kseg columns (a multiple of 32; the last one
+// may be shorter).  splits = 1: not cut, kseg = k.
+struct KSplit {
+  int splits, kseg;
+};
+inline KSplit k_split(int k, int64_t want) {
+  if (want < 2) return {1, k};
+  const int kseg = (int)((k + want - 1) / want + 31) / 32 * 32;
+  return {(k + kseg - 1) / kseg, kseg};
+}
+// 64 x 64 tiles: about two CTAs per SM, at least 128 columns each.  An empty k
+// (a product with alpha = 0) is not cut.
+inline KSplit tile_split(int tiles, int k) {
+  return k_split(k, std::min(2 * 148 / tiles, k / 128));
+}
+// Few columns, 32 rows per CTA: about eight CTAs per SM, at least 512 columns
+// each.
+inline KSplit skinny_split(int m, int k) {
+  return k_split(k, std::min<int64_t>((int64_t)8 * 148 * 32 / m + 1, (k + 511) / 512));
 }
 
 }  // namespace rfp

@@ -1,6 +1,7 @@
 // layout_checks.cpp — TEST-ONLY host entry points for the index arithmetic
-// of the single-read symmetric matrix-vector kernel (symv_layout.h) and the
-// routing of few-column products (gemm_route.h), run without a GPU.
+// of the single-read symmetric matrix-vector kernel (symv_layout.h), the
+// routing of few-column products and the split of k (gemm_route.h), run
+// without a GPU.
 #include <cstdint>
 #include <vector>
 
@@ -82,6 +83,15 @@ int hs_skinny_route(int m, int n, int k, int k2, int a_tri, int b_tri, int c_low
   out[4] = s.use ? r.m : 0;
   out[5] = s.use ? r.n : 0;
   out[6] = s.use ? r.k : 0;
+  return 0;
+}
+
+// The split of k for `tiles` 64 x 64 tiles (few = 0) or m rows of a few-column
+// product (few = 1).  out: splits, columns per split.
+int hs_k_split(int few, int size, int k, int* out) {
+  const KSplit s = few ? skinny_split(size, k) : tile_split(size, k);
+  out[0] = s.splits;
+  out[1] = s.kseg;
   return 0;
 }
 
