@@ -11,6 +11,7 @@
 
 #include "../../include/curfp.h"
 #include "context.h"
+#include "func_attr.h"
 #include "k_pack.cuh"
 #include "k_refine.cuh"
 #include "k_symv.cuh"
@@ -55,17 +56,6 @@ inline int read_info(curfpHandle_t h, int* info, int* err) {
 int symm_launch(curfpHandle_t h, const Geometry& g, const float* A, const float* X,
                 int64_t ldx, float* Y, int64_t ldy, int nrhs, float alpha, float beta);
 
-inline bool symm_attr() {
-  static bool done = false;
-  if (!done) {
-    if (cudaFuncSetAttribute(rfp::kref::symm_acc64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             rfp::kref::SYMM_SMEM) != cudaSuccess)
-      return false;
-    done = true;
-  }
-  return true;
-}
-
 // Flags a zero on the diagonal of the factor (the condition on which the
 // reference's SPOTRI reports failure, src/curfp_spftri.cu:318,326).
 template <typename T>
@@ -106,7 +96,8 @@ curfpStatus_t pack(curfpHandle_t h, int transr, int lower, int n, const T* src,
 
 int symm_launch(curfpHandle_t h, const Geometry& g, const float* A, const float* X,
                 int64_t ldx, float* Y, int64_t ldy, int nrhs, float alpha, float beta) {
-  if (!symm_attr()) return 4;
+  static rfp::OncePerDevice attr;
+  if (!rfp::smem_attr(attr, h->device, rfp::kref::symm_acc64, rfp::kref::SYMM_SMEM)) return 4;
   const int n = g.n;
   const int bx = (n + rfp::kref::TB - 1) / rfp::kref::TB, by = (nrhs + rfp::kref::TB - 1) / rfp::kref::TB;
   int split = 1;

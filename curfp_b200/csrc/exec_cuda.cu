@@ -6,6 +6,7 @@
 #include <type_traits>
 
 #include "context.h"
+#include "func_attr.h"
 #include "k_chain.cuh"
 #include "k_chain1.cuh"
 #include "k_chol.cuh"
@@ -378,24 +379,14 @@ int CudaExecT<float>::gemm(const GemmProb* p, int count) {
   return launch_gemm<float, 64, 64>(p, count, abort_, ctx_, may_allocate());
 }
 
-namespace {
-// Opt a kernel into more than 48 KB of dynamic shared memory (once per
-// instantiation).
-template <typename K>
-bool smem_attr(K kernel, int bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) ==
-         cudaSuccess;
-}
-}  // namespace
-
 template <typename T>
 int CudaExecT<T>::potrf_adj_tile(ViewT<T> L, ViewT<T> G, int n) {
   if (n <= 0) return 0;
   if (n > ktile::T) return 3;
   ProfScope ps(ctx_->prof, ctx_->stream, K_POTRF, 2.0 * n * (double)n * n / 3.0, 0);
   constexpr int smem = ktile::adj_smem<T>();
-  static const bool attr = smem_attr(ktile::potrf_adj_tile<T>, smem);
-  if (!attr) return 4;
+  static OncePerDevice attr;
+  if (!smem_attr(attr, ctx_->device, ktile::potrf_adj_tile<T>, smem)) return 4;
   ktile::potrf_adj_tile<T><<<1, ktile::ADJ_THREADS, smem, ctx_->stream>>>(L, G, n);
   ++ctx_->launches;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
@@ -423,8 +414,8 @@ int launch_chol(curfpContext* ctx, ViewT<T> V11, ViewT<T> V21, ViewT<T> V22, int
   a.err = ctx->d_info + 1;
   a.info_base = info_base;
   constexpr int smem = kchol::smem_bytes<T>();
-  static const bool attr = smem_attr(kchol::chol_wave<T>, smem);
-  if (!attr) return 4;
+  static OncePerDevice attr;
+  if (!smem_attr(attr, ctx->device, kchol::chol_wave<T>, smem)) return 4;
   const double n = (double)n1 + n2, m = panel ? n2 : 0;
   ProfScope ps(ctx->prof, ctx->stream, K_POTRF,
                panel ? (n1 / 3.0 + m) * n1 * n1 : n * n * n / 3.0, 0);
@@ -479,8 +470,8 @@ int CudaExecT<T>::trtri_batch(const ViewT<T>* L, const int* n, int count, T* W) 
   b.W = W;
   ProfScope ps(ctx_->prof, ctx_->stream, K_TRTRI, flops, 0);
   constexpr int smem = ktile::trtri_smem<T>();
-  static const bool attr = smem_attr(ktile::trtri_blocks<T>, smem);
-  if (!attr) return 4;
+  static OncePerDevice attr;
+  if (!smem_attr(attr, ctx_->device, ktile::trtri_blocks<T>, smem)) return 4;
   ktile::trtri_blocks<T><<<blocks, ktile::TRTRI_THREADS, smem, ctx_->stream>>>(b, abort_);
   ++ctx_->launches;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
@@ -523,8 +514,8 @@ int CudaExecT<T>::trtri_block(ViewT<T> L, int n) {
   a.err = ctx_->d_info + 1;
   a.abort_flag = abort_;
   constexpr int smem = ktri::smem_bytes<T>();
-  static const bool attr = smem_attr(ktri::inverse_wave<T>, smem);
-  if (!attr) return 4;
+  static OncePerDevice attr;
+  if (!smem_attr(attr, ctx_->device, ktri::inverse_wave<T>, smem)) return 4;
   ProfScope ps(ctx_->prof, ctx_->stream, K_TRTRI, (double)n * n * n / 3, 0);
   ps.shape(n, n, n, tiles);
   ktri::inverse_wave<T><<<tiles, ktri::THR, smem, ctx_->stream>>>(a);
@@ -588,8 +579,8 @@ int launch_wave(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int n, Vie
   // does not share its SM with another CTA's accumulation.
   constexpr int smem = ktrsv::smem_bytes<T, NC>();
   constexpr int smem_one = ktrsv::smem_limit<T, NC>();
-  static const bool attr = smem_attr(ktrsv::trsm_wave<T, NC>, smem_one);
-  if (!attr) return 4;
+  static OncePerDevice attr;
+  if (!smem_attr(attr, ctx->device, ktrsv::trsm_wave<T, NC>, smem_one)) return 4;
   const int smem_launch = nchunk <= 2 ? smem_one : smem;
   ProfScope ps(ctx->prof, ctx->stream, K_TRSV, (double)n * n * m,
                (double)n * n * sizeof(T) / 2.0);
@@ -623,8 +614,8 @@ int launch_chain(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int n, Vi
   if (cudaMemsetAsync(a.sync, 0, words * sizeof(int), ctx->stream) != cudaSuccess) return 4;
   a.err = ctx->d_info + 1;
   a.abort_flag = abort_flag;
-  static const bool attr = smem_attr(kchain::trsm_chain<T, NC>, C::SMEM);
-  if (!attr) return 4;
+  static OncePerDevice attr;
+  if (!smem_attr(attr, ctx->device, kchain::trsm_chain<T, NC>, C::SMEM)) return 4;
   ProfScope ps(ctx->prof, ctx->stream, K_TRSV, (double)n * n * m, (double)n * n * sizeof(T) / 2.0);
   ps.shape(n, m, n, (int)tiles);
   const int grid = (a.nblk + kchain::CS - 1) / kchain::CS * a.nchunk * kchain::CS;
@@ -686,8 +677,8 @@ int launch_solve_tiles(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int
   a.err = ctx->d_info + 1;
   a.abort_flag = abort_flag;
   constexpr int smem = ktri::smem_bytes<T>();
-  static const bool attr = smem_attr(ktri::solve_tiles<T>, smem);
-  if (!attr) return 4;
+  static OncePerDevice attr;
+  if (!smem_attr(attr, ctx->device, ktri::solve_tiles<T>, smem)) return 4;
   ProfScope ps(ctx->prof, ctx->stream, K_TRSV, (double)n * n * m, (double)n * n * sizeof(T) / 2.0);
   ps.shape(n, m, n, (int)tiles);
   if (lower > 0) {
@@ -753,8 +744,9 @@ int wave_wait_selftest(curfpContext* ctx) {
       cudaSuccess)
     return 4;
   constexpr int smem = ktrsv::smem_bytes<float, 8>();
-  static const bool attr = smem_attr(ktrsv::trsm_wave<float, 8>, ktrsv::smem_limit<float, 8>());
-  if (!attr) return 4;
+  static OncePerDevice attr;
+  if (!smem_attr(attr, ctx->device, ktrsv::trsm_wave<float, 8>, ktrsv::smem_limit<float, 8>()))
+    return 4;
   ktrsv::trsm_wave<float, 8><<<nblk - 1, 256, smem, ctx->stream>>>(
       View{Lp, n, 1}, n, View{Bp, 1, n}, m, 1.0f, Wp, sync, ctx->d_info + 1, nullptr);
   ++ctx->launches;
@@ -769,9 +761,8 @@ int launch_trsm_wave_fixed(curfpContext* ctx, const int* abort_flag, View L, int
   const size_t words = 1 + (size_t)nblk * nchunk;
   if (words > sync_words) return 3;
   if (cudaMemsetAsync(sync, 0, words * 4, ctx->stream) != cudaSuccess) return 4;
-  if (cudaFuncSetAttribute(ktrsv::trsm_wave<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           ktrsv::smem_limit<float>()) != cudaSuccess)
-    return 4;
+  static OncePerDevice attr;
+  if (!smem_attr(attr, ctx->device, ktrsv::trsm_wave<float>, ktrsv::smem_limit<float>())) return 4;
   ProfScope ps(ctx->prof, ctx->stream, K_TRSV, (double)n * n * m, (double)n * n * 2.0);
   ktrsv::trsm_wave<float><<<nblk * nchunk, 256, ktrsv::SMEM, ctx->stream>>>(
       L, n, B, m, alpha, W, sync, ctx->d_info + 1, abort_flag);

@@ -7,6 +7,7 @@
 #include <mutex>
 
 #include "context.h"
+#include "func_attr.h"
 #include "k_tc.cuh"
 
 namespace rfp {
@@ -180,13 +181,8 @@ int tc_slab(curfpContext* ctx, const int* abort_flag, View A, int arows, int ama
   b.b_scale = sb.scale;
   b.abort_flag = abort_flag;
   b.err_flag = ctx->d_info + 1;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(ktc::tc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             ktc::SMEM_BYTES) != cudaSuccess)
-      return 4;
-    attr_set = true;
-  }
+  static OncePerDevice attr;
+  if (!smem_attr(attr, ctx->device, ktc::tc_gemm_kernel, ktc::SMEM_BYTES)) return 4;
   const int sms = sm_count(ctx);
   const int grid = tiles < sms ? tiles : sms;  // persistent: one CTA per SM
   ProfScope ps(ctx->prof, ctx->stream, K_TC_GEMM, flops, 0);

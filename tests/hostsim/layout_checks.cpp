@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "func_attr.h"
 #include "gemm_route.h"
 #include "symv_layout.h"
 
@@ -92,6 +93,23 @@ int hs_k_split(int few, int size, int k, int* out) {
   const KSplit s = few ? skinny_split(size, k) : tile_split(size, k);
   out[0] = s.splits;
   out[1] = s.kseg;
+  return 0;
+}
+
+// A setting made once per device: `calls` devices are asked for in order, the
+// setter fails for the fail_at-th run (-1: never).  out[i]: result of call i,
+// + 2 if the setter ran.
+int hs_once_per_device(int calls, const int* device, int fail_at, int* out) {
+  OncePerDevice once;
+  int runs = 0;
+  for (int i = 0; i < calls; ++i) {
+    bool ran = false;
+    const bool ok = once(device[i], [&] {
+      ran = true;
+      return runs++ != fail_at;
+    });
+    out[i] = (ok ? 1 : 0) + (ran ? 2 : 0);
+  }
   return 0;
 }
 
