@@ -213,14 +213,18 @@ curfpStatus_t curfpReleaseWorkspace(curfpHandle_t handle) {
 
 curfpStatus_t curfpDiagWaitTimeout(curfpHandle_t handle, int* err_code) {
   if (!handle || !err_code) return CURFP_STATUS_INVALID_VALUE;
-  if (!reset_info(handle)) return CURFP_STATUS_EXECUTION_FAILED;
   // The error word is read and cleared by the same check that every routine
   // with bounded waits runs before it returns (status.cuh), so the code
   // reported here is the one a real solve would surface, and later calls on
-  // this handle do not inherit it.
-  rfp::status::WaitCheck wc(handle);
-  const int rc = wc.finish(rfp::wave_wait_selftest(handle));
-  *err_code = wc.err;
+  // this handle do not inherit it.  Every kernel has to report the code.
+  int rc = 0;
+  *err_code = 5;
+  for (int kind = 0; kind < rfp::kWaitSelftests && *err_code == 5; ++kind) {
+    if (!reset_info(handle)) return CURFP_STATUS_EXECUTION_FAILED;
+    rfp::status::WaitCheck wc(handle);
+    rc = wc.finish(rfp::wait_selftest(handle, kind));
+    *err_code = wc.err;
+  }
   return status_of(rc);
 }
 

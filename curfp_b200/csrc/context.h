@@ -22,6 +22,7 @@ struct curfpContext {
   cudaMemPool_t pool = nullptr;  // the handle's workspace pool
   int math = 1;            // contraction arithmetic of the drop-in routines (curfpSetMathMode)
   long long wait_launches = 0;  // kernels with bounded waits launched (status.cuh)
+  int skip_tickets = 0;    // self-test: first tickets of a waiting kernel that no CTA takes
   int* d_info = nullptr;   // [0]: INT_MAX = no pivot failure; [1]: kernel error code
   void* ws = nullptr;      // TRSM diagonal-block inverses and other scratch
   size_t ws_bytes = 0;
@@ -130,10 +131,11 @@ int tc_contract_masked(curfpContext* ctx, const int* abort_flag, View A, int aro
 // (cleared here on the stream); no allocation.
 int launch_trsm_wave_fixed(curfpContext* ctx, const int* abort_flag, View L, int n, View B,
                            int m, float alpha, const float* W, int* sync, size_t sync_words);
-// Bounded-wait self-test of the wavefront solve (exec_cuda.cu): launches a
-// solve whose first block row never runs; its dependents time out (~2 s) and
-// set error code 5 in ctx->d_info[1].
-int wave_wait_selftest(curfpContext* ctx);
+// Bounded-wait self-tests (exec_cuda.cu), kind 0 to kWaitSelftests - 1: each
+// launches one waiting kernel whose first ticket no CTA takes; the CTAs that
+// depend on it time out (~2 s) and set error code 5 in ctx->d_info[1].
+constexpr int kWaitSelftests = 2;
+int wait_selftest(curfpContext* ctx, int kind);
 // Whether a contraction of this size goes to the tensor-core path.
 bool tc_worthwhile(int m, int n, int k);
 // Whether a contraction with operands of at most `rows` rows stages its

@@ -565,6 +565,17 @@ int CudaExecT<T>::lauum_block(ViewT<T> L, int n) {
 }
 
 namespace {
+// Clears a waiting kernel's flags and its ticket counter, which the self-test
+// starts behind the tickets it leaves out.
+int clear_sync(curfpContext* ctx, void* flags, size_t bytes, int* ticket) {
+  if (cudaMemsetAsync(flags, 0, bytes, ctx->stream) != cudaSuccess) return 4;
+  if (ctx->skip_tickets &&
+      cudaMemcpyAsync(ticket, &ctx->skip_tickets, sizeof(int), cudaMemcpyHostToDevice,
+                      ctx->stream) != cudaSuccess)
+    return 4;
+  return 0;
+}
+
 // The wavefront solve with NC right-hand-side columns per CTA.
 template <typename T, int NC>
 int launch_wave(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int n, ViewT<T> B, int m,
@@ -637,15 +648,14 @@ int launch_chain1(curfpContext* ctx, const int* abort_flag, View L, int n, View 
   a.ws = static_cast<unsigned long long*>(
       grow_buffer(ctx, &ctx->tsv, &ctx->tsv_bytes, words * sizeof(unsigned long long)));
   if (!a.ws) return 2;
-  if (cudaMemsetAsync(a.ws, 0, words * sizeof(unsigned long long), ctx->stream) != cudaSuccess)
-    return 4;
   a.sync = reinterpret_cast<int*>(a.ws + words - 1);
+  if (clear_sync(ctx, a.ws, words * sizeof(unsigned long long), a.sync)) return 4;
   a.err = ctx->d_info + 1;
   a.abort_flag = abort_flag;
   ProfScope ps(ctx->prof, ctx->stream, K_TRSV, (double)n * n, (double)n * n * 2.0);
   ps.shape(n, 1, n, a.nblk);
-  kchain1::chain1<<<(a.nblk + kchain::CS - 1) / kchain::CS * kchain::CS, kchain1::THR, 0,
-                    ctx->stream>>>(a);
+  const int clusters = (a.nblk + kchain::CS - 1) / kchain::CS - ctx->skip_tickets;
+  kchain1::chain1<<<clusters * kchain::CS, kchain1::THR, 0, ctx->stream>>>(a);
   ++ctx->launches;
   ++ctx->wait_launches;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
@@ -728,7 +738,7 @@ template class CudaExecT<double>;
 // at 1), so block rows 1 and 2 wait on a flag that nothing sets.  Their
 // waits give up after ~2 s, set error code 5 in the handle's error word and
 // return; the caller reads the word.  All buffers are zeroed first.
-int wave_wait_selftest(curfpContext* ctx) {
+static int wave_wait_selftest(curfpContext* ctx) {
   constexpr int n = 3 * ktrsv::NB, m = 1, nblk = 3;
   const size_t fl = (size_t)n * n + n * m + (size_t)nblk * kInvStride;
   const size_t bytes = fl * sizeof(float) + (1 + nblk) * sizeof(int);
@@ -752,6 +762,25 @@ int wave_wait_selftest(curfpContext* ctx) {
   ++ctx->launches;
   ++ctx->wait_launches;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+
+// Bounded-wait self-test of one kernel through its ordinary launch: a solve
+// with 16 block rows whose first ticket (its first eight rows) no CTA takes.
+// The operands are zeros and live in a buffer that no launch takes scratch from.
+int wait_selftest(curfpContext* ctx, int kind) {
+  if (kind == 0) return wave_wait_selftest(ctx);
+  constexpr int n = 1024, nblk = n / kTrsmLeaf;
+  const size_t fl = (size_t)n * n + n + (size_t)nblk * kInvStride;
+  float* L = static_cast<float*>(
+      grow_buffer(ctx, &ctx->wsg, &ctx->wsg_bytes, fl * sizeof(float)));
+  if (!L) return 2;
+  if (cudaMemsetAsync(L, 0, fl * sizeof(float), ctx->stream) != cudaSuccess) return 4;
+  float* B = L + (size_t)n * n;
+  CudaExec ex(ctx);
+  ctx->skip_tickets = 1;
+  const int rc = ex.trsm_wave(View{L, n, 1}, n, View{B, 1, n}, 1, 1.0f, B + n);
+  ctx->skip_tickets = 0;
+  return rc;
 }
 
 int launch_trsm_wave_fixed(curfpContext* ctx, const int* abort_flag, View L, int n, View B,

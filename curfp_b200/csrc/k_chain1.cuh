@@ -15,7 +15,8 @@
 // 8-column kernel, 108 us so, 2048 rows 48 and 30 us.
 //
 // Waits are bounded (~2 s); a wait that runs out records an error code and the
-// CTA goes on with what it has, so that every hand-off still takes place.
+// CTA goes on with what it has, so that every hand-off still takes place.  No
+// word is poisoned: the error word alone says that the result is void.
 #pragma once
 #include <climits>
 #include <cstdint>
@@ -266,7 +267,14 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(THR, 1) chain1(cons
   }
   // No CTA leaves while another may still write to its shared memory: every
   // send precedes the barrier, and every block sent here has been waited for.
+  // The barrier orders a send, not its arrival, so a thread that stopped
+  // waiting waits (bounded) for what was sent now.
   kchain::cluster_barrier();
+  if (late && j < g.nblk) {
+    const uint64_t t0 = ktrsv::gtimer();
+    for (int s = 0; s < rank; ++s)
+      while (!try_parity(su32(&in[s]), 0) && ktrsv::gtimer() - t0 < 1000000ull) {}
+  }
 }
 
 }  // namespace kchain1

@@ -413,11 +413,12 @@ curfpStatus_t curfpReleaseWorkspace(curfpHandle_t handle);
 curfpStatus_t curfpGetKernelLaunchCount(curfpHandle_t handle, long long *count);
 
 /* Self-test of the kernels' failure detection (no counterpart in the
- * reference): launches a small wavefront solve whose first block row never
- * runs, so the CTAs of the next rows wait on a flag that nothing sets.  Their
- * waits are bounded: after ~2 s they record error code 5 in the handle's
- * error word and return, and the call reports CURFP_STATUS_EXECUTION_FAILED
- * with *err_code = 5.  The context stays usable.  Takes ~2 s. */
+ * reference): launches small solves whose first block rows never run, one
+ * after the other, so the CTAs of the next rows wait on a flag that nothing
+ * sets.  Their waits are bounded: after ~2 s they record error code 5 in the
+ * handle's error word and return, and the call reports
+ * CURFP_STATUS_EXECUTION_FAILED with *err_code = 5 when every one of them did.
+ * The context stays usable.  Takes ~2 s per kernel. */
 curfpStatus_t curfpDiagWaitTimeout(curfpHandle_t handle, int *err_code);
 
 /* Optional kernel timing: when enabled, every kernel this handle launches is
