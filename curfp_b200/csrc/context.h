@@ -134,7 +134,7 @@ int launch_trsm_wave_fixed(curfpContext* ctx, const int* abort_flag, View L, int
 // Bounded-wait self-tests (exec_cuda.cu), kind 0 to kWaitSelftests - 1: each
 // launches one waiting kernel whose first ticket no CTA takes; the CTAs that
 // depend on it time out (~2 s) and set error code 5 in ctx->d_info[1].
-constexpr int kWaitSelftests = 2;
+constexpr int kWaitSelftests = 6;
 int wait_selftest(curfpContext* ctx, int kind);
 // Whether a contraction of this size goes to the tensor-core path.
 bool tc_worthwhile(int m, int n, int k);

@@ -51,6 +51,17 @@ T* CudaExecT<T>::workspace(size_t count) {
 
 namespace {
 
+// Clears a waiting kernel's flags and its ticket counter, which the self-test
+// starts behind the tickets it leaves out.
+int clear_sync(curfpContext* ctx, void* flags, size_t bytes, int* ticket) {
+  if (cudaMemsetAsync(flags, 0, bytes, ctx->stream) != cudaSuccess) return 4;
+  if (ctx->skip_tickets &&
+      cudaMemcpyAsync(ticket, &ctx->skip_tickets, sizeof(int), cudaMemcpyHostToDevice,
+                      ctx->stream) != cudaSuccess)
+    return 4;
+  return 0;
+}
+
 template <typename T, int BM, int BN>
 int launch_gemm(const GemmProbT<T>* p, int count, const int* abort_flag,
                 curfpContext* ctx, bool alloc = false) {
@@ -409,7 +420,7 @@ int launch_chol(curfpContext* ctx, ViewT<T> V11, ViewT<T> V21, ViewT<T> V22, int
       grow_buffer(ctx, &ctx->ws, &ctx->ws_bytes, tiles * kchol::TILE * sizeof(T)));
   a.sync = static_cast<int*>(grow_buffer(ctx, &ctx->tsv, &ctx->tsv_bytes, words * sizeof(int)));
   if (!a.ws || !a.sync) return 2;
-  if (cudaMemsetAsync(a.sync, 0, words * sizeof(int), ctx->stream) != cudaSuccess) return 4;
+  if (clear_sync(ctx, a.sync, words * sizeof(int), a.sync)) return 4;
   a.info = ctx->d_info;
   a.err = ctx->d_info + 1;
   a.info_base = info_base;
@@ -420,7 +431,8 @@ int launch_chol(curfpContext* ctx, ViewT<T> V11, ViewT<T> V21, ViewT<T> V22, int
   ProfScope ps(ctx->prof, ctx->stream, K_POTRF,
                panel ? (n1 / 3.0 + m) * n1 * n1 : n * n * n / 3.0, 0);
   ps.shape(n1, n2, panel ? 1 : 0, (int)tiles);
-  kchol::chol_wave<T><<<kchol::cta_count(a.nb, a.nbf), kchol::threads<T>(), smem, ctx->stream>>>(a);
+  const int ctas = kchol::cta_count(a.nb, a.nbf) - ctx->skip_tickets;
+  kchol::chol_wave<T><<<ctas, kchol::threads<T>(), smem, ctx->stream>>>(a);
   ++ctx->launches;
   ++ctx->wait_launches;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
@@ -510,7 +522,7 @@ int CudaExecT<T>::trtri_block(ViewT<T> L, int n) {
                                      (size_t)tiles * ktri::TILE * sizeof(T)));
   a.sync = static_cast<int*>(grow_buffer(ctx_, &ctx_->tsv, &ctx_->tsv_bytes, words * sizeof(int)));
   if (!a.ws || !a.sync) return 2;
-  if (cudaMemsetAsync(a.sync, 0, words * sizeof(int), ctx_->stream) != cudaSuccess) return 4;
+  if (clear_sync(ctx_, a.sync, words * sizeof(int), a.sync)) return 4;
   a.err = ctx_->d_info + 1;
   a.abort_flag = abort_;
   constexpr int smem = ktri::smem_bytes<T>();
@@ -518,7 +530,7 @@ int CudaExecT<T>::trtri_block(ViewT<T> L, int n) {
   if (!smem_attr(attr, ctx_->device, ktri::inverse_wave<T>, smem)) return 4;
   ProfScope ps(ctx_->prof, ctx_->stream, K_TRTRI, (double)n * n * n / 3, 0);
   ps.shape(n, n, n, tiles);
-  ktri::inverse_wave<T><<<tiles, ktri::THR, smem, ctx_->stream>>>(a);
+  ktri::inverse_wave<T><<<tiles - ctx_->skip_tickets, ktri::THR, smem, ctx_->stream>>>(a);
   ktri::store_inverse<T><<<tiles, ktri::THR, 0, ctx_->stream>>>(L, n, a.ws, abort_);
   ctx_->launches += 2;
   ++ctx_->wait_launches;
@@ -565,17 +577,6 @@ int CudaExecT<T>::lauum_block(ViewT<T> L, int n) {
 }
 
 namespace {
-// Clears a waiting kernel's flags and its ticket counter, which the self-test
-// starts behind the tickets it leaves out.
-int clear_sync(curfpContext* ctx, void* flags, size_t bytes, int* ticket) {
-  if (cudaMemsetAsync(flags, 0, bytes, ctx->stream) != cudaSuccess) return 4;
-  if (ctx->skip_tickets &&
-      cudaMemcpyAsync(ticket, &ctx->skip_tickets, sizeof(int), cudaMemcpyHostToDevice,
-                      ctx->stream) != cudaSuccess)
-    return 4;
-  return 0;
-}
-
 // The wavefront solve with NC right-hand-side columns per CTA.
 template <typename T, int NC>
 int launch_wave(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int n, ViewT<T> B, int m,
@@ -584,7 +585,7 @@ int launch_wave(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int n, Vie
   const size_t words = 1 + (size_t)nblk * nchunk;
   int* sync = static_cast<int*>(grow_buffer(ctx, &ctx->tsv, &ctx->tsv_bytes, words * 4));
   if (!sync) return 2;
-  if (cudaMemsetAsync(sync, 0, words * 4, ctx->stream) != cudaSuccess) return 4;
+  if (clear_sync(ctx, sync, words * 4, sync)) return 4;
   // With at most two chunks the chain of block rows sets the time: the
   // shared-memory request is padded to one CTA per SM, so the chain's product
   // does not share its SM with another CTA's accumulation.
@@ -596,7 +597,7 @@ int launch_wave(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int n, Vie
   ProfScope ps(ctx->prof, ctx->stream, K_TRSV, (double)n * n * m,
                (double)n * n * sizeof(T) / 2.0);
   ps.shape(n, m, n, nblk * nchunk);
-  ktrsv::trsm_wave<T, NC><<<nblk * nchunk, 256, smem_launch, ctx->stream>>>(
+  ktrsv::trsm_wave<T, NC><<<nblk * nchunk - ctx->skip_tickets, 256, smem_launch, ctx->stream>>>(
       L, n, B, m, alpha, W, sync, ctx->d_info + 1, abort_flag);
   ++ctx->launches;
   ++ctx->wait_launches;
@@ -622,15 +623,15 @@ int launch_chain(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int n, Vi
       grow_buffer(ctx, &ctx->wst, &ctx->wst_bytes, tiles * C::XT * sizeof(T)));
   a.sync = static_cast<int*>(grow_buffer(ctx, &ctx->tsv, &ctx->tsv_bytes, words * sizeof(int)));
   if (!a.ws || !a.sync) return 2;
-  if (cudaMemsetAsync(a.sync, 0, words * sizeof(int), ctx->stream) != cudaSuccess) return 4;
+  if (clear_sync(ctx, a.sync, words * sizeof(int), a.sync)) return 4;
   a.err = ctx->d_info + 1;
   a.abort_flag = abort_flag;
   static OncePerDevice attr;
   if (!smem_attr(attr, ctx->device, kchain::trsm_chain<T, NC>, C::SMEM)) return 4;
   ProfScope ps(ctx->prof, ctx->stream, K_TRSV, (double)n * n * m, (double)n * n * sizeof(T) / 2.0);
   ps.shape(n, m, n, (int)tiles);
-  const int grid = (a.nblk + kchain::CS - 1) / kchain::CS * a.nchunk * kchain::CS;
-  kchain::trsm_chain<T, NC><<<grid, kchain::THR, C::SMEM, ctx->stream>>>(a);
+  const int clusters = (a.nblk + kchain::CS - 1) / kchain::CS * a.nchunk - ctx->skip_tickets;
+  kchain::trsm_chain<T, NC><<<clusters * kchain::CS, kchain::THR, C::SMEM, ctx->stream>>>(a);
   ++ctx->launches;
   ++ctx->wait_launches;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
@@ -683,7 +684,7 @@ int launch_solve_tiles(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int
   a.ws = ws + (size_t)lower * ktri::TILE;
   a.sync = static_cast<int*>(grow_buffer(ctx, &ctx->tsv, &ctx->tsv_bytes, words * sizeof(int)));
   if (!ws || !a.sync) return 2;
-  if (cudaMemsetAsync(a.sync, 0, words * sizeof(int), ctx->stream) != cudaSuccess) return 4;
+  if (clear_sync(ctx, a.sync, words * sizeof(int), a.sync)) return 4;
   a.err = ctx->d_info + 1;
   a.abort_flag = abort_flag;
   constexpr int smem = ktri::smem_bytes<T>();
@@ -695,7 +696,7 @@ int launch_solve_tiles(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int
     ktri::pack_lower<T><<<lower, ktri::THR, 0, ctx->stream>>>(L, n, ws, abort_flag);
     ++ctx->launches;
   }
-  ktri::solve_tiles<T><<<(int)tiles, ktri::THR, smem, ctx->stream>>>(a);
+  ktri::solve_tiles<T><<<(int)tiles - ctx->skip_tickets, ktri::THR, smem, ctx->stream>>>(a);
   ++ctx->launches;
   ++ctx->wait_launches;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
@@ -733,52 +734,31 @@ int CudaExecT<T>::trsm_wave(ViewT<T> L, int n, ViewT<T> B, int m, T alpha, const
 template class CudaExecT<float>;
 template class CudaExecT<double>;
 
-// Bounded-wait self-test: a wavefront solve of three 64-row block rows in
-// which the CTA of block row 0 is never launched (the ticket counter starts
-// at 1), so block rows 1 and 2 wait on a flag that nothing sets.  Their
-// waits give up after ~2 s, set error code 5 in the handle's error word and
-// return; the caller reads the word.  All buffers are zeroed first.
-static int wave_wait_selftest(curfpContext* ctx) {
-  constexpr int n = 3 * ktrsv::NB, m = 1, nblk = 3;
-  const size_t fl = (size_t)n * n + n * m + (size_t)nblk * kInvStride;
-  const size_t bytes = fl * sizeof(float) + (1 + nblk) * sizeof(int);
-  char* buf = static_cast<char*>(grow_buffer(ctx, &ctx->ws, &ctx->ws_bytes, bytes));
-  if (!buf) return 2;
-  if (cudaMemsetAsync(buf, 0, bytes, ctx->stream) != cudaSuccess) return 4;
-  float* Lp = reinterpret_cast<float*>(buf);
-  float* Bp = Lp + (size_t)n * n;
-  float* Wp = Bp + n * m;
-  int* sync = reinterpret_cast<int*>(Wp + (size_t)nblk * kInvStride);
-  static const int one = 1;
-  if (cudaMemcpyAsync(sync, &one, sizeof(int), cudaMemcpyHostToDevice, ctx->stream) !=
-      cudaSuccess)
-    return 4;
-  constexpr int smem = ktrsv::smem_bytes<float, 8>();
-  static OncePerDevice attr;
-  if (!smem_attr(attr, ctx->device, ktrsv::trsm_wave<float, 8>, ktrsv::smem_limit<float, 8>()))
-    return 4;
-  ktrsv::trsm_wave<float, 8><<<nblk - 1, 256, smem, ctx->stream>>>(
-      View{Lp, n, 1}, n, View{Bp, 1, n}, m, 1.0f, Wp, sync, ctx->d_info + 1, nullptr);
-  ++ctx->launches;
-  ++ctx->wait_launches;
-  return cudaGetLastError() == cudaSuccess ? 0 : 4;
-}
-
-// Bounded-wait self-test of one kernel through its ordinary launch: a solve
-// with 16 block rows whose first ticket (its first eight rows) no CTA takes.
-// The operands are zeros and live in a buffer that no launch takes scratch from.
+// Bounded-wait self-test of one waiting kernel through its ordinary launch, the
+// CTAs of its first ticket (the first tile; in the two cluster chains the first
+// eight block rows) left out.  The operands are zeros and live in a buffer
+// that no launch takes scratch from.
 int wait_selftest(curfpContext* ctx, int kind) {
-  if (kind == 0) return wave_wait_selftest(ctx);
-  constexpr int n = 1024, nblk = n / kTrsmLeaf;
-  const size_t fl = (size_t)n * n + n + (size_t)nblk * kInvStride;
+  constexpr int n = 1024, m = 4096, nblk = n / kTrsmLeaf;
+  constexpr size_t nb = (size_t)192 * m;  // right-hand sides: 1024 x 9, 192 x 600, 192 x 4096
+  constexpr size_t fl = (size_t)n * n + nb + (size_t)nblk * kInvStride;
   float* L = static_cast<float*>(
       grow_buffer(ctx, &ctx->wsg, &ctx->wsg_bytes, fl * sizeof(float)));
   if (!L) return 2;
   if (cudaMemsetAsync(L, 0, fl * sizeof(float), ctx->stream) != cudaSuccess) return 4;
   float* B = L + (size_t)n * n;
+  const float* W = B + nb;
   CudaExec ex(ctx);
   ctx->skip_tickets = 1;
-  const int rc = ex.trsm_wave(View{L, n, 1}, n, View{B, 1, n}, 1, 1.0f, B + n);
+  int rc = 3;
+  switch (kind) {
+    case 0: rc = ex.trsm_wave(View{L, n, 1}, n, View{B, 1, n}, 1, 1.0f, W); break;    // chain1
+    case 1: rc = ex.trsm_wave(View{L, n, 1}, n, View{B, 1, n}, 9, 1.0f, W); break;    // trsm_chain
+    case 2: rc = ex.trsm_wave(View{L, n, 1}, 192, View{B, 1, 192}, 600, 1.0f, W); break;  // trsm_wave
+    case 3: rc = ex.trsm_wave(View{L, n, 1}, 192, View{B, 1, 192}, m, 1.0f, W); break;  // solve_tiles
+    case 4: rc = ex.trtri_block(View{L, n, 1}, 192); break;                          // inverse_wave
+    case 5: rc = ex.potrf_tile(View{L, n, 1}, 192, 0); break;                        // chol_wave
+  }
   ctx->skip_tickets = 0;
   return rc;
 }

@@ -174,8 +174,9 @@ def release_workspace() -> None:
 
 
 def diag_wait_timeout() -> tuple:
-    """Self-test of the kernels' bounded waits (~2 s each): solves whose first
-    block rows never run; returns (status, error code), which is
+    """Self-test of the kernels' bounded waits (~2 s each, ~12 s in all): the
+    solve, inverse and Cholesky kernels on small problems whose first tile
+    never runs; returns (status, error code), which is
     (CURFP_STATUS_EXECUTION_FAILED, 5) when the waits give up as designed."""
     h = _get_handle()
     code = ctypes.c_int(0)

@@ -413,12 +413,13 @@ curfpStatus_t curfpReleaseWorkspace(curfpHandle_t handle);
 curfpStatus_t curfpGetKernelLaunchCount(curfpHandle_t handle, long long *count);
 
 /* Self-test of the kernels' failure detection (no counterpart in the
- * reference): launches small solves whose first block rows never run, one
- * after the other, so the CTAs of the next rows wait on a flag that nothing
- * sets.  Their waits are bounded: after ~2 s they record error code 5 in the
- * handle's error word and return, and the call reports
- * CURFP_STATUS_EXECUTION_FAILED with *err_code = 5 when every one of them did.
- * The context stays usable.  Takes ~2 s per kernel. */
+ * reference): launches each kernel that hands tiles on through flags (the
+ * solves, the triangular inverse, the Cholesky factorization) on a small
+ * problem whose first tile never runs, so that the others wait on a flag that
+ * nothing sets.  Their waits are bounded: after ~2 s they record error code 5
+ * in the handle's error word and return, and the call reports
+ * CURFP_STATUS_EXECUTION_FAILED with *err_code = 5 when every kernel did.  The
+ * context stays usable.  Takes ~2 s per kernel, ~12 s in all. */
 curfpStatus_t curfpDiagWaitTimeout(curfpHandle_t handle, int *err_code);
 
 /* Optional kernel timing: when enabled, every kernel this handle launches is
