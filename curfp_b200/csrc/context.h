@@ -61,8 +61,8 @@ constexpr int kCholRfpRows = 4096;
 // digits are relative to its largest element, and an inverse factor's rows
 // have a dominant diagonal (n = 6001 inverse, error against FP64: 1.8e-5 with
 // 2048-row blocks on the tensor cores, 5e-7 with the diagonal kept apart,
-// 1.9e-7 this way).  1024 against 512 rows: 6.2 against 7.5 ms for that
-// inverse (25.6 ms with 64-row leaves).
+// 1.3e-7 this way, 1.8e-7 with 64-row leaves).  1024 against 512 rows: 6.2
+// against 7.5 ms for that inverse (25.6 ms with 64-row leaves).
 constexpr int kTriRows = 2048;
 constexpr int kLeafRows = 1024;
 constexpr int kSolveTilesRhs = 4096;  // FP32 leaf solves: columns from which throughput counts

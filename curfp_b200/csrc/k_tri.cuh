@@ -5,6 +5,9 @@
 // CTA waits only on smaller tickets and no co-residency is needed.  CTA (i, c),
 // c <= i:
 //   M_ic = W_i (I_ic - sum_{c<=k<i} L_ik M_kc),   W_i = inv(L_ii).
+// The term k = c, which holds M's dominant diagonal tile, is subtracted by
+// itself: a running sum that starts with it rounds every later term against it
+// (inverse at n = 2000: error 2.0e-7 so, 1.7e-7 apart, at 1% of the time).
 // Other CTAs read L throughout, so the result stays in the published tiles
 // until store_inverse writes it over L.
 //
@@ -147,7 +150,23 @@ __global__ void __launch_bounds__(THR, sizeof(T) == 4 ? 2 : 1) inverse_wave(cons
       if (ready) load_x(k + 1);
       ktrsv::cp_commit();
       // rows of the register tile: M's columns, columns: L's rows
-      product8<NB, LDL, NB / G>(acc, Xs + par * TILE, Ls + par * NB * LDL, grp * (NB / G), u);
+      if (k == c) {  // the dominant term goes to T by itself
+        const int tr = tid & 15, tc = tid >> 4;
+        T s[4][4];
+        product4<NB, LDL>(s, Xs, Ls, 0, NB / 4, tr, tc);
+#pragma unroll 1
+        for (int q = 1; q < 4; ++q) {
+          T o[4][4];
+          product4<NB, LDL>(o, Xs, Ls, q * (NB / 4), (q + 1) * (NB / 4), tr, tc);
+#pragma unroll
+          for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) s[a][b] += o[a][b];
+        }
+        put4<LDL, true>(Ts, s, tr, tc);
+      } else {
+        product8<NB, LDL, NB / G>(acc, Xs + par * TILE, Ls + par * NB * LDL, grp * (NB / G), u);
+      }
       if (more && !ready) {
         if (warp == 0) wait(k + 1, &sh_known[2]);
         __syncthreads();
@@ -158,25 +177,27 @@ __global__ void __launch_bounds__(THR, sizeof(T) == 4 ? 2 : 1) inverse_wave(cons
       }
     }
     // T -= the groups' partial sums, which meet in the operand buffers
-    __syncthreads();
-    store8(Ls + grp * TILE, acc, u);
-    __syncthreads();
+    if (i > c + 1) {
+      __syncthreads();
+      store8(Ls + grp * TILE, acc, u);
+      __syncthreads();
 #pragma unroll
-    for (int w = 0; w < TILE / 4 / THR; ++w) {
-      const int e = (tid + THR * w) * 4;
-      T* t = Ts + (e / NB) * LDL + e % NB;
-      T s[4], v[4];
-      lds4(Ls + e, s);
+      for (int w = 0; w < TILE / 4 / THR; ++w) {
+        const int e = (tid + THR * w) * 4;
+        T* t = Ts + (e / NB) * LDL + e % NB;
+        T s[4], v[4];
+        lds4(Ls + e, s);
 #pragma unroll
-      for (int q = 1; q < G; ++q) {
-        lds4(Ls + q * TILE + e, v);
+        for (int q = 1; q < G; ++q) {
+          lds4(Ls + q * TILE + e, v);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) s[r] += v[r];
+          for (int r = 0; r < 4; ++r) s[r] += v[r];
+        }
+        lds4(t, v);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) v[r] -= s[r];
+        sts4(t, v);
       }
-      lds4(t, v);
-#pragma unroll
-      for (int r = 0; r < 4; ++r) v[r] -= s[r];
-      sts4(t, v);
     }
   }
   ktrsv::cp_commit();
