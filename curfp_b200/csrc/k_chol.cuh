@@ -189,6 +189,24 @@ __device__ __forceinline__ int factor32(T* s, T* raw, int bar0) {
   for (int k = 0; k < 32; ++k) s[k * NB + lane] = a[k];
   return fail;
 }
+// The pivots whose reciprocal is a normal number.
+template <typename T> struct Pivot;
+template <> struct Pivot<float> { static constexpr float lo = 0x1p-126f, hi = 0x1p125f; };
+template <> struct Pivot<double> { static constexpr double lo = 0x1p-1022, hi = 0x1p1021; };
+
+// inverse32 for pivots of any size: 1 / d_j, infinite for a subnormal d_j, is
+// never formed; 2^64 or 2^-64 of it goes to the column instead.
+template <typename T>
+__device__ __noinline__ void inverse32_any(T* w, const T* raw) {
+  T* x = w + (threadIdx.x & 31) * LDW;
+  for (int k = 0; k < 32; ++k) x[k] = k == (threadIdx.x & 31) ? T(1) : T(0);
+  for (int j = 0; j < 32; ++j) {
+    const T d = raw[j * 32 + j], r = rsqrt_newton(d), u = x[j] * r;
+    const T s = d < T(1) ? T(0x1p64) : T(0x1p-64), v = u * (T(1) / s) * r;
+    x[j] = u;
+    for (int k = j + 1; k < 32; ++k) x[k] = fma(raw[j * 32 + k] * s, -v, x[k]);
+  }
+}
 // The warp that follows factor32: lane = column of the inverse, written to w
 // (column-major, stride LDW, zeros above the diagonal).  Column j of the
 // factor is raw_j / sqrt(d_j), so x_j /= sqrt(d_j), then
@@ -199,9 +217,14 @@ __device__ __forceinline__ void inverse32(T* w, const T* raw, int bar0) {
   T x[32];
 #pragma unroll
   for (int k = 0; k < 32; ++k) x[k] = k == lane ? T(1) : T(0);
+  bool any = false;  // a pivot whose reciprocal is not normal
   each_column<0>([&](auto jc) {
     constexpr int j = decltype(jc)::value;
     if ((j & 7) == 0) bar_sync_id<64>(bar0 + (j >> 3));
+    if (j == 24) {  // every pivot is there
+      const T d = raw[lane * 33];
+      any = __any_sync(0xffffffffu, !(d >= Pivot<T>::lo && d <= Pivot<T>::hi));
+    }
     T lk[32];
 #pragma unroll
     for (int v4 = j / 4; v4 < 8; ++v4)
@@ -211,6 +234,7 @@ __device__ __forceinline__ void inverse32(T* w, const T* raw, int bar0) {
     x[j] = u;
     axpy<j + 1>(x, -v, lk);
   });
+  if (any) return inverse32_any(w, raw);
 #pragma unroll
   for (int k = 0; k < 32; k += 4) {
     const T v[4] = {x[k], x[k + 1], x[k + 2], x[k + 3]};
