@@ -65,7 +65,6 @@ constexpr int kCholRfpRows = 4096;
 // against 7.5 ms for that inverse (25.6 ms with 64-row leaves).
 constexpr int kTriRows = 2048;
 constexpr int kLeafRows = 1024;
-constexpr int kSolveTilesRhs = 4096;  // FP32 leaf solves: columns from which throughput counts
 
 // The CUDA executor for FP32 (SIMT and split-BF16 tensor-core contractions)
 // and FP64 (SIMT DFMA) element types.

@@ -69,8 +69,7 @@ constexpr int kTrsmLeaf = 64;    // TRSM diagonal blocks (inverted, then multipl
 constexpr int kInvStride = 2 * kTrsmLeaf * kTrsmLeaf;
 constexpr int kTriTile = 64;     // trtri / lauum tiles
 constexpr int kAdjTile = 64;     // Cholesky-adjoint diagonal tiles
-constexpr int kTrsvMaxRhs = 512; // wavefront solve for at most this many RHS
-constexpr int kWaveLeaf = 512;   // recursive TRSM hands blocks <= this to the wavefront solve
+constexpr int kTrsvMaxRhs = 512; // one-launch solves for at most this many RHS (solve_route.h)
 constexpr int kNotSupported = -1;
 
 template <typename T>

@@ -16,6 +16,7 @@
 #include "k_tile.cuh"
 #include "k_tri.cuh"
 #include "k_trsv.cuh"
+#include "solve_route.h"
 
 namespace rfp {
 
@@ -703,31 +704,21 @@ int launch_solve_tiles(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int
 }
 }  // namespace
 
-// Up to kTrsvMaxRhs right-hand sides (FP64 128): the chain inside clusters, in
-// chunks as narrow as the throughput allows, since the chain's step shrinks
-// with the chunk while the products' cost per column grows: 8 columns up to
-// 256 (block row, chunk) pairs, 16 up to 512, else 32 (8192 rows, 16 / 64 / 128
-// columns: 8 wide 190 / 510 / 970 us, 16 wide 262 / 390 / 690 us, 32 wide 400 /
-// 420 / 600 us; FP64 8 wide); a single FP32 column has its own kernel.  More right-hand sides keep every SM busy
-// (n = 512 leaves of the recursion): 64-column chunks handed on through L2, in
-// FP32 from kSolveTilesRhs columns on by the kernel made for throughput (512
-// rows, 2048 / 4096 / 16384 columns: 70 / 88 / 208 us, there 77 / 79 / 148).
+// The kernels' choice: solve_route.h.
 template <typename T>
 int CudaExecT<T>::trsm_wave(ViewT<T> L, int n, ViewT<T> B, int m, T alpha, const T* W) {
   if (n <= 0 || m <= 0) return 0;
-  const int nblk = (n + kTrsmLeaf - 1) / kTrsmLeaf;
-  if (m <= (sizeof(T) == 4 ? kTrsvMaxRhs : 128)) {
-    if constexpr (sizeof(T) == 4) {
-      if (m == 1) return launch_chain1(ctx_, abort_, L, n, B, alpha, W);
-      if ((int64_t)nblk * ((m + 15) / 16) > 512)
-        return launch_chain<T, 32>(ctx_, abort_, L, n, B, m, alpha, W);
-      if ((int64_t)nblk * ((m + 7) / 8) > 256)
-        return launch_chain<T, 16>(ctx_, abort_, L, n, B, m, alpha, W);
+  const SolveKernel kernel = solve_kernel(sizeof(T) == 4, n, m);
+  if constexpr (sizeof(T) == 4) {
+    switch (kernel) {
+      case SOLVE_CHAIN1: return launch_chain1(ctx_, abort_, L, n, B, alpha, W);
+      case SOLVE_CHAIN16: return launch_chain<T, 16>(ctx_, abort_, L, n, B, m, alpha, W);
+      case SOLVE_CHAIN32: return launch_chain<T, 32>(ctx_, abort_, L, n, B, m, alpha, W);
+      case SOLVE_TILES: return launch_solve_tiles<T>(ctx_, abort_, L, n, B, m, alpha, W);
+      default: break;
     }
-    return launch_chain<T, 8>(ctx_, abort_, L, n, B, m, alpha, W);
   }
-  if constexpr (sizeof(T) == 4)
-    if (m >= kSolveTilesRhs) return launch_solve_tiles<T>(ctx_, abort_, L, n, B, m, alpha, W);
+  if (kernel == SOLVE_CHAIN8) return launch_chain<T, 8>(ctx_, abort_, L, n, B, m, alpha, W);
   return launch_wave<T, 64>(ctx_, abort_, L, n, B, m, alpha, W);
 }
 

@@ -7,6 +7,7 @@
 // src/curfp_ssfrk.cpp:193-209), and every dense sub-problem is then solved
 // recursively on the views.
 #include "engine.h"
+#include "solve_route.h"
 
 namespace rfp {
 namespace plan {
@@ -47,9 +48,8 @@ int trsm_rec(ExecT<T>& ex, ViewT<T> L, int n, ViewT<T> B, int m, Scalar<T> alpha
     p.inplace = 1;
     return ex.gemm(&p, 1);
   }
-  // Leaves go to the wavefront solve, small ones, so that most of the work is
-  // in the (tensor-core) GEMM updates.
-  if (n <= kWaveLeaf) {
+  // Leaves are one launch (solve_route.h).
+  if (n <= solve_leaf_rows(m)) {
     int rc = ex.trsm_wave(L, n, B, m, alpha, Wb);
     if (rc != kNotSupported) return rc;
   }
@@ -81,10 +81,7 @@ int trsm_with(ExecT<T>& ex, ViewT<T> L, int n, ViewT<T> B, int m, Scalar<T> alph
     if ((rc = ex.trtri_blocks(L, n, kTrsmLeaf, w))) return rc;
     W = w;
   }
-  // One wavefront launch for few right-hand sides: up to kTrsvMaxRhs the
-  // recursion's launches cost more than its products save, tensor cores or not
-  // (n = 4096, 400 columns: 0.5 ms against 0.9 ms).
-  if (m <= kTrsvMaxRhs) {
+  if (solve_in_one_launch(n, m, math)) {
     rc = ex.trsm_wave(L, n, B, m, alpha, W);
     if (rc != kNotSupported) return rc;
   }

@@ -8,6 +8,7 @@
 #include "engine.h"
 #include "func_attr.h"
 #include "gemm_route.h"
+#include "solve_route.h"
 #include "symv_layout.h"
 
 using namespace rfp;
@@ -93,6 +94,15 @@ int hs_k_split(int few, int size, int k, int* out) {
   const KSplit s = few ? skinny_split(size, k) : tile_split(size, k);
   out[0] = s.splits;
   out[1] = s.kseg;
+  return 0;
+}
+
+// The solve of an n-row triangle with m right-hand sides.  out: one launch (or
+// the recursion), rows of the recursion's leaves, kernel of a launch.
+int hs_solve_route(int fp32, int n, int m, int math, int* out) {
+  out[0] = solve_in_one_launch(n, m, math);
+  out[1] = solve_leaf_rows(m);
+  out[2] = solve_kernel(fp32 != 0, n, m);
   return 0;
 }
 
