@@ -419,9 +419,13 @@ int launch_chol(curfpContext* ctx, ViewT<T> V11, ViewT<T> V21, ViewT<T> V22, int
   const size_t tiles = (size_t)kchol::tile_count(a.nb, a.nbf), words = 1 + tiles;
   a.ws = static_cast<T*>(
       grow_buffer(ctx, &ctx->ws, &ctx->ws_bytes, tiles * kchol::TILE * sizeof(T)));
-  a.sync = static_cast<int*>(grow_buffer(ctx, &ctx->tsv, &ctx->tsv_bytes, words * sizeof(int)));
-  if (!a.ws || !a.sync) return 2;
-  if (clear_sync(ctx, a.sync, words * sizeof(int), a.sync)) return 4;
+  if (!a.ws) return 2;
+  const int ctas = kchol::cta_count(a.nb, a.nbf) - ctx->skip_tickets;
+  if (ctas > 1) {
+    a.sync = static_cast<int*>(grow_buffer(ctx, &ctx->tsv, &ctx->tsv_bytes, words * sizeof(int)));
+    if (!a.sync) return 2;
+    if (clear_sync(ctx, a.sync, words * sizeof(int), a.sync)) return 4;
+  }
   a.info = ctx->d_info;
   a.err = ctx->d_info + 1;
   a.info_base = info_base;
@@ -432,7 +436,6 @@ int launch_chol(curfpContext* ctx, ViewT<T> V11, ViewT<T> V21, ViewT<T> V22, int
   ProfScope ps(ctx->prof, ctx->stream, K_POTRF,
                panel ? (n1 / 3.0 + m) * n1 * n1 : n * n * n / 3.0, 0);
   ps.shape(n1, n2, panel ? 1 : 0, (int)tiles);
-  const int ctas = kchol::cta_count(a.nb, a.nbf) - ctx->skip_tickets;
   kchol::chol_wave<T><<<ctas, kchol::threads<T>(), smem, ctx->stream>>>(a);
   ++ctx->launches;
   ++ctx->wait_launches;

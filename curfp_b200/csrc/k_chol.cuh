@@ -72,7 +72,8 @@ struct Args {
   int n1, n2, nb1, nb;  // orders, tiles of the first block, tiles in all
   int nbf;              // tile columns factored: nb, or nb1
   T* ws;                // published tiles (tile_index; W_i at (i, i))
-  int* sync;            // [0] ticket, [1 + tile] flags (0 not ready, 1 ready, -1 poisoned)
+  int* sync;            // [0] ticket, [1 + tile] flags (0 not ready, 1 ready, -1 poisoned);
+                        // nullptr for a single CTA
   int* info;            // pivot failures (INT_MAX: none)
   int* err;             // wait timeouts
   int info_base;
@@ -323,7 +324,7 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
   const int warp = tid >> 5, lane = tid & 31;
   constexpr int NW = THR / 32;
   if (tid == 0) {
-    sh_ticket = atomicAdd(g.sync, 1);
+    sh_ticket = g.sync ? atomicAdd(g.sync, 1) : 0;
     sh_fail = 0;
   }
   const bool abort = g.info && *g.info != INT_MAX;
@@ -344,7 +345,7 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
     __syncthreads();
     if (tid == 0) {
       if (c >= 0) ktrsv::st_release(&flags[tidx(i, c)], -1);
-      if (diag) ktrsv::st_release(&flags[tidx(i, i)], -1);
+      if (diag && g.sync) ktrsv::st_release(&flags[tidx(i, i)], -1);
     }
   };
   if (__syncthreads_or(abort)) return poison();  // a pivot failed earlier
@@ -514,6 +515,8 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
   // beside L10 (n = 2000: 414 against 440 us); in FP64 the factor is longer and
   // both ways take the same time, so its order stays.
   constexpr bool kBeside = sizeof(T) == 4;
+  // A tile of up to 32 rows has no second half: zeros and the identity in W.
+  const bool half = sr <= 32;
   const bool shadow = (warp & 3) >= 2;
   const int st = ((warp >> 2) * 2 + (warp & 1)) * 32 + lane;
 #pragma unroll 1
@@ -569,7 +572,7 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
       }
     }
     __syncthreads();
-    if (sh_fail || h == 1) break;
+    if (sh_fail || h == 1 || half) break;
     // Half of the groups: L10 = S10 inv(D0)^T; with kBeside the others
     // S11 -= X1 X1^T.  Then S11 -= L10 L10^T.
     T o[4][4];
@@ -593,9 +596,16 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
     }
     __syncthreads();
   }
+  if (half) {
+    for (int e = tid; e < 32 * 64; e += THR) {
+      const int cc = e & 63, r = 32 + (e >> 6);
+      Ws[cc * LDW + r] = cc == r ? T(1) : T(0);
+    }
+    __syncthreads();
+  }
   if (!sh_fail) {
     // W10 = -inv(D1) P
-    for (int c0 = warp * 2; c0 < 32; c0 += NW * 2) {
+    for (int c0 = half ? 32 : warp * 2; c0 < 32; c0 += NW * 2) {
       T o[2] = {T(0), T(0)};
 #pragma unroll
       for (int k = 0; k < 32; k += 4) {
@@ -622,11 +632,11 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
       sts4(wout + e * 4, v);
     }
     __syncthreads();
-    if (tid == 0) ktrsv::st_release(&flags[tidx(i, i)], 1);
+    if (tid == 0 && g.sync) ktrsv::st_release(&flags[tidx(i, i)], 1);
   } else if (tid == 0) {
     const int col0 = i >= g.nb1 ? g.n1 + (i - g.nb1) * NB : i * NB;
     atomicMin(g.info, g.info_base + col0 + sh_fail);
-    ktrsv::st_release(&flags[tidx(i, i)], -1);
+    if (g.sync) ktrsv::st_release(&flags[tidx(i, i)], -1);
   }
   if (c >= 0) store_matrix(Xs, xv, xr, xc, false);
   store_matrix(Ss, sv, sr, sr, true);
