@@ -211,14 +211,15 @@ __device__ __noinline__ void inverse32_any(T* w, const T* raw) {
 // The warp that follows factor32: lane = column of the inverse, written to w
 // (column-major, stride LDW, zeros above the diagonal).  Column j of the
 // factor is raw_j / sqrt(d_j), so x_j /= sqrt(d_j), then
-// x_i -= raw_ij (x_j / sqrt(d_j)).
+// x_i -= raw_ij (x_j / sqrt(d_j)).  Returns whether a pivot asks for
+// inverse32_any instead.
 template <typename T>
-__device__ __forceinline__ void inverse32(T* w, const T* raw, int bar0) {
+__device__ __forceinline__ bool inverse32(T* w, const T* raw, int bar0) {
   const int lane = threadIdx.x & 31;
   T x[32];
 #pragma unroll
   for (int k = 0; k < 32; ++k) x[k] = k == lane ? T(1) : T(0);
-  bool any = false;  // a pivot whose reciprocal is not normal
+  bool any = false;
   each_column<0>([&](auto jc) {
     constexpr int j = decltype(jc)::value;
     if ((j & 7) == 0) bar_sync_id<64>(bar0 + (j >> 3));
@@ -235,12 +236,12 @@ __device__ __forceinline__ void inverse32(T* w, const T* raw, int bar0) {
     x[j] = u;
     axpy<j + 1>(x, -v, lk);
   });
-  if (any) return inverse32_any(w, raw);
 #pragma unroll
   for (int k = 0; k < 32; k += 4) {
     const T v[4] = {x[k], x[k + 1], x[k + 2], x[k + 3]};
     sts4(w + lane * LDW + k, v);
   }
+  return any;
 }
 
 // Tile (row tile i, column tile j) of the matrix as a view and its extents.
@@ -318,14 +319,15 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
   T* Ts = B0 + 2 * TILE;
   T* Ss = Ts + TILE;
   T* Ws = Ss + TILE;  // W_i, column stride LDW
-  __shared__ int sh_ticket, sh_known[3], sh_state, sh_fail;
+  __shared__ int sh_ticket, sh_known[3], sh_state;
+  __shared__ int2 sh_odd;  // 1 + a failing column of the diagonal tile, pivots out of range
   constexpr int THR = threads<T>(), G = groups<T>();
   const int tid = threadIdx.x, grp = tid >> 6, u = tid & 63;
   const int warp = tid >> 5, lane = tid & 31;
   constexpr int NW = THR / 32;
   if (tid == 0) {
     sh_ticket = g.sync ? atomicAdd(g.sync, 1) : 0;
-    sh_fail = 0;
+    sh_odd = make_int2(0, 0);
   }
   const bool abort = g.info && *g.info != INT_MAX;
   __syncthreads();
@@ -518,14 +520,16 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
   // A tile of up to 32 rows has no second half: zeros and the identity in W.
   const bool half = sr <= 32;
   const bool shadow = (warp & 3) >= 2;
+  int fail = 0;  // 1 + the failing column
   const int st = ((warp >> 2) * 2 + (warp & 1)) * 32 + lane;
 #pragma unroll 1
   for (int h = 0; h < 2; ++h) {  // one copy of the code (instruction cache)
     if (warp == 0) {
       const int f = factor32(Ss + h * (32 * NB + 32), raw, 2 + 4 * h);
-      if (lane == 0 && f) sh_fail = 32 * h + f;
+      if (lane == 0 && f) sh_odd.x = 32 * h + f;
     } else if (warp == 1) {
-      inverse32(Ws + h * (32 * LDW + 32), raw, 2 + 4 * h);
+      const bool any = inverse32(Ws + h * (32 * LDW + 32), raw, 2 + 4 * h);
+      if (lane == 0) sh_odd.y = any;
     } else if (h == 0 && shadow) {
       if (c >= 0) {
         T o[4][4];
@@ -572,7 +576,13 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
       }
     }
     __syncthreads();
-    if (sh_fail || h == 1 || half) break;
+    const int2 odd = sh_odd;
+    fail = odd.x;
+    if (odd.y) {
+      if (warp == 1) inverse32_any(Ws + h * (32 * LDW + 32), raw);
+      __syncthreads();
+    }
+    if (fail || h == 1 || half) break;
     // Half of the groups: L10 = S10 inv(D0)^T; with kBeside the others
     // S11 -= X1 X1^T.  Then S11 -= L10 L10^T.
     T o[4][4];
@@ -603,7 +613,7 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
     }
     __syncthreads();
   }
-  if (!sh_fail) {
+  if (!fail) {
     // W10 = -inv(D1) P
     for (int c0 = half ? 32 : warp * 2; c0 < 32; c0 += NW * 2) {
       T o[2] = {T(0), T(0)};
@@ -635,7 +645,7 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
     if (tid == 0 && g.sync) ktrsv::st_release(&flags[tidx(i, i)], 1);
   } else if (tid == 0) {
     const int col0 = i >= g.nb1 ? g.n1 + (i - g.nb1) * NB : i * NB;
-    atomicMin(g.info, g.info_base + col0 + sh_fail);
+    atomicMin(g.info, g.info_base + col0 + fail);
     if (g.sync) ktrsv::st_release(&flags[tidx(i, i)], -1);
   }
   if (c >= 0) store_matrix(Xs, xv, xr, xc, false);
