@@ -115,7 +115,13 @@ int launch_gemm(const GemmProbT<T>* p, int count, const int* abort_flag,
   }
   ProfScope ps(ctx->prof, st, K_SGEMM, flops, 0);
   ps.shape(b.p[0].m, b.p[0].n, b.p[0].k + b.p[0].k2, tiles);
-  kgemm::sgemm_batch<T, BM, BN><<<dim3(tiles, splits), kgemm::kThreads, 0, st>>>(b);
+  bool blocked = false;
+  if constexpr (BM == 64) {
+    blocked = cnt == 1 && !q0.k2 && (q0.a_tri || q0.b_tri);
+    if (blocked) kgemm::sgemm_batch<T, BM, BN, true><<<tiles, kgemm::kThreads, 0, st>>>(b);
+  }
+  if (!blocked)
+    kgemm::sgemm_batch<T, BM, BN><<<dim3(tiles, splits), kgemm::kThreads, 0, st>>>(b);
   ++ctx->launches;
   if (splits > 1) {
     kgemm::split_reduce<T, BM, BN><<<tiles, kgemm::kThreads, 0, st>>>(b, splits);

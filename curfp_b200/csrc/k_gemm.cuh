@@ -253,7 +253,7 @@ __device__ __forceinline__ void k_range(int k, int a_tri, int b_tri, int m0, int
   if (ke < kb) ke = kb;
 }
 
-template <typename T, int BM, int BN>
+template <typename T, int BM, int BN, bool kBlocked = false>
 __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && BM >= 128) ? 1 : 2)
     sgemm_batch(const Batch<T> batch) {
   if (batch.abort_flag && *batch.abort_flag != INT_MAX) return;
@@ -286,14 +286,13 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && BM >= 128) ? 1 : 
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = T(0);
 
-  // 64 x 64 tiles of masked products (the triangular multiplies and L^T L
-  // products of up to 1024 rows that the inverse ends in): the sums of each
-  // 128 columns meet in a second set of registers, so that no element is one
-  // chain of 1024 roundings (inverse, n = 2000: error 1.7e-7 without, 9.5e-8
-  // with; 1.4e-7 for the recursion down to 64 rows; n = 6001 5.8 -> 5.9 ms).
-  constexpr bool kBlocked = BM == 64;
+  // kBlocked (64 x 64 tiles of a single masked product: the triangular
+  // multiplies and L^T L products of up to 1024 rows that the inverse ends in):
+  // the sums of each 128 columns meet in a second set of registers, so that no
+  // element is one chain of 1024 roundings (inverse, n = 2000: error 1.7e-7
+  // without, 9.5e-8 with; 1.4e-7 for the recursion down to 64 rows; n = 6001
+  // 5.8 -> 5.9 ms).
   constexpr int kFlush = 128 / BK;
-  const bool blocked = kBlocked && (P.a_tri | P.b_tri);
   T sum[kBlocked ? TM : 1][kBlocked ? TN : 1];
   if constexpr (kBlocked) {
 #pragma unroll
@@ -303,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && BM >= 128) ? 1 : 
   }
   auto flush = [&](int kt) {
     if constexpr (kBlocked) {
-      if (!blocked || kt % kFlush != kFlush - 1) return;
+      if (kt % kFlush != kFlush - 1) return;
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
