@@ -649,20 +649,21 @@ static curfpStatus_t sfmv_impl(curfpHandle_t handle, curfpOperation_t transr,
         a, part, y + oy, incy, *alpha, *beta);
     handle->launches += 2;
     return ok_launch() ? CURFP_STATUS_SUCCESS : CURFP_STATUS_EXECUTION_FAILED;
+  } else {
+    const rfp::ksymv::Parts P = rfp::ksymv::parts(n);
+    T* part = static_cast<T*>(rfp::grow_buffer(handle, &handle->ws, &handle->ws_bytes,
+                                               (size_t)(P.n_row + P.n_col) * sizeof(T)));
+    if (!part) return CURFP_STATUS_ALLOC_FAILED;
+    const double nt = (double)n * (n + 1) / 2;
+    rfp::ProfScope ps(handle->prof, handle->stream, rfp::K_SGEMM, 4.0 * nt, sizeof(T) * nt);
+    rfp::ksymv::symv_tiles<T>
+        <<<(unsigned)rfp::ksymv::strips_before(P.tiles), rfp::ksymv::kThreads, 0, handle->stream>>>(
+            g, arf, x + ox, incx, part);
+    rfp::ksymv::symv_reduce<T><<<P.tiles, rfp::ksymv::kThreads, 0, handle->stream>>>(
+        n, part, y + oy, incy, *alpha, *beta);
+    handle->launches += 2;
+    return ok_launch() ? CURFP_STATUS_SUCCESS : CURFP_STATUS_EXECUTION_FAILED;
   }
-  const rfp::ksymv::Parts P = rfp::ksymv::parts(n);
-  T* part = static_cast<T*>(rfp::grow_buffer(handle, &handle->ws, &handle->ws_bytes,
-                                             (size_t)(P.n_row + P.n_col) * sizeof(T)));
-  if (!part) return CURFP_STATUS_ALLOC_FAILED;
-  const double nt = (double)n * (n + 1) / 2;
-  rfp::ProfScope ps(handle->prof, handle->stream, rfp::K_SGEMM, 4.0 * nt, sizeof(T) * nt);
-  rfp::ksymv::symv_tiles<T>
-      <<<(unsigned)rfp::ksymv::strips_before(P.tiles), rfp::ksymv::kThreads, 0, handle->stream>>>(
-          g, arf, x + ox, incx, part);
-  rfp::ksymv::symv_reduce<T><<<P.tiles, rfp::ksymv::kThreads, 0, handle->stream>>>(
-      n, part, y + oy, incy, *alpha, *beta);
-  handle->launches += 2;
-  return ok_launch() ? CURFP_STATUS_SUCCESS : CURFP_STATUS_EXECUTION_FAILED;
 }
 
 curfpStatus_t curfpSsfmv(curfpHandle_t handle, curfpOperation_t transr, curfpFillMode_t uplo,

@@ -587,27 +587,22 @@ int CudaExecT<T>::lauum_block(ViewT<T> L, int n) {
 }
 
 namespace {
-// The wavefront solve with NC right-hand-side columns per CTA.
-template <typename T, int NC>
+// The wavefront solve, 64 right-hand-side columns per CTA.
+template <typename T>
 int launch_wave(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int n, ViewT<T> B, int m,
                 T alpha, const T* W) {
-  const int nblk = (n + ktrsv::NB - 1) / ktrsv::NB, nchunk = (m + NC - 1) / NC;
+  const int nblk = (n + ktrsv::NB - 1) / ktrsv::NB, nchunk = (m + ktrsv::NB - 1) / ktrsv::NB;
   const size_t words = 1 + (size_t)nblk * nchunk;
   int* sync = static_cast<int*>(grow_buffer(ctx, &ctx->tsv, &ctx->tsv_bytes, words * 4));
   if (!sync) return 2;
   if (clear_sync(ctx, sync, words * 4, sync)) return 4;
-  // With at most two chunks the chain of block rows sets the time: the
-  // shared-memory request is padded to one CTA per SM, so the chain's product
-  // does not share its SM with another CTA's accumulation.
-  constexpr int smem = ktrsv::smem_bytes<T, NC>();
-  constexpr int smem_one = ktrsv::smem_limit<T, NC>();
+  constexpr int smem = ktrsv::smem_bytes<T>();
   static OncePerDevice attr;
-  if (!smem_attr(attr, ctx->device, ktrsv::trsm_wave<T, NC>, smem_one)) return 4;
-  const int smem_launch = nchunk <= 2 ? smem_one : smem;
+  if (!smem_attr(attr, ctx->device, ktrsv::trsm_wave<T>, smem)) return 4;
   ProfScope ps(ctx->prof, ctx->stream, K_TRSV, (double)n * n * m,
                (double)n * n * sizeof(T) / 2.0);
   ps.shape(n, m, n, nblk * nchunk);
-  ktrsv::trsm_wave<T, NC><<<nblk * nchunk - ctx->skip_tickets, 256, smem_launch, ctx->stream>>>(
+  ktrsv::trsm_wave<T><<<nblk * nchunk - ctx->skip_tickets, 256, smem, ctx->stream>>>(
       L, n, B, m, alpha, W, sync, ctx->d_info + 1, abort_flag);
   ++ctx->launches;
   ++ctx->wait_launches;
@@ -728,7 +723,7 @@ int CudaExecT<T>::trsm_wave(ViewT<T> L, int n, ViewT<T> B, int m, T alpha, const
     }
   }
   if (kernel == SOLVE_CHAIN8) return launch_chain<T, 8>(ctx_, abort_, L, n, B, m, alpha, W);
-  return launch_wave<T, 64>(ctx_, abort_, L, n, B, m, alpha, W);
+  return launch_wave<T>(ctx_, abort_, L, n, B, m, alpha, W);
 }
 
 template class CudaExecT<float>;
@@ -770,10 +765,11 @@ int launch_trsm_wave_fixed(curfpContext* ctx, const int* abort_flag, View L, int
   const size_t words = 1 + (size_t)nblk * nchunk;
   if (words > sync_words) return 3;
   if (cudaMemsetAsync(sync, 0, words * 4, ctx->stream) != cudaSuccess) return 4;
+  constexpr int smem = ktrsv::smem_bytes<float>();
   static OncePerDevice attr;
-  if (!smem_attr(attr, ctx->device, ktrsv::trsm_wave<float>, ktrsv::smem_limit<float>())) return 4;
+  if (!smem_attr(attr, ctx->device, ktrsv::trsm_wave<float>, smem)) return 4;
   ProfScope ps(ctx->prof, ctx->stream, K_TRSV, (double)n * n * m, (double)n * n * 2.0);
-  ktrsv::trsm_wave<float><<<nblk * nchunk, 256, ktrsv::SMEM, ctx->stream>>>(
+  ktrsv::trsm_wave<float><<<nblk * nchunk, 256, smem, ctx->stream>>>(
       L, n, B, m, alpha, W, sync, ctx->d_info + 1, abort_flag);
   ++ctx->launches;
   ++ctx->wait_launches;

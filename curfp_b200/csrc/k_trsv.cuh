@@ -37,33 +37,14 @@ constexpr int NB = 64;
 constexpr int LDL = NB + 4;
 constexpr uint64_t WAIT_NS = 2000000000ull;
 
-// Right-hand-side chunk of one CTA: NC columns, each thread a TR x TC
-// register tile of the 64 x NC block; EPT elements of an X tile per thread;
-// X / T tiles with row stride LDX.  NC = 64 for many right-hand sides, NC = 8
-// for few (a single vector keeps the chain's per-block product small).
-template <int NC> struct Chunk;
-template <> struct Chunk<64> {
-  static constexpr int TR = 4, TC = 4, EPT = 16, LDX = NB + 4;  // 16-byte reads along a row
-};
-template <> struct Chunk<8> {
-  static constexpr int TR = 2, TC = 1, EPT = 2, LDX = 8;
-};
-constexpr int LDX = Chunk<64>::LDX;
+// X / T tiles have row stride LDX (16-byte reads along a row); a thread owns a
+// 4 x 4 register tile of the 64 x 64 block and EPT elements of an X tile.
+constexpr int LDX = NB + 4, EPT = 16;
 
-// Ls[2], Ws (L tiles; W_j; M_j reuses Ls[0]) and Xs[2], Ts (X tiles; B_jc / T);
-// 8-column chunks add the partial sums of their k-split products.
-constexpr int LDP = NB + 1;  // row stride of the partial sums
-template <int NC> constexpr int kparts() { return NC == 8 ? 4 * 8 * LDP : 0; }
-template <typename T, int NC = 64>
+// Ls[2], Ws (L tiles; W_j; M_j reuses Ls[0]) and Xs[2], Ts (X tiles; B_jc / T).
+template <typename T>
 constexpr int smem_bytes() {
-  return (3 * NB * LDL + 3 * NB * Chunk<NC>::LDX + kparts<NC>()) * (int)sizeof(T);
-}
-constexpr int SMEM = smem_bytes<float>();
-// The dynamic shared-memory limit set on every instantiation: its own need,
-// or at least 116 KB so that a launch may ask for one CTA per SM.
-template <typename T, int NC = 64>
-constexpr int smem_limit() {
-  return smem_bytes<T, NC>() > 116 * 1024 ? smem_bytes<T, NC>() : 116 * 1024;
+  return (3 * NB * LDL + 3 * NB * LDX) * (int)sizeof(T);
 }
 
 __device__ __forceinline__ int ld_acquire(const int* p) {
@@ -109,27 +90,26 @@ __device__ __forceinline__ void load_tile(T* s, ViewT<T> v, int rows, int cols) 
     cp1(s + b * LD + a, ok ? v.p + (int64_t)a * v.rs + (int64_t)b * v.cs : v.p, ok);
   }
 }
-// Tile of B / X (64 x NC, written by CTAs of this launch): L2-only loads
+// Tile of B / X (64 x 64, written by CTAs of this launch): L2-only loads
 // into registers (ld.global.cg), stored to shared memory by store_regs.
-template <int NC, typename T>
-__device__ __forceinline__ void load_regs(T (&r)[Chunk<NC>::EPT], ViewT<T> v, int rows,
-                                          int cols) {
+template <typename T>
+__device__ __forceinline__ void load_regs(T (&r)[EPT], ViewT<T> v, int rows, int cols) {
   const bool rowcont = (v.cs == 1 || v.cs == -1) && !(v.rs == 1 || v.rs == -1);
 #pragma unroll
-  for (int u = 0; u < Chunk<NC>::EPT; ++u) {
+  for (int u = 0; u < EPT; ++u) {
     const int e = threadIdx.x + 256 * u;
-    const int a = rowcont ? e / NC : e % NB, b = rowcont ? e % NC : e / NB;
+    const int a = rowcont ? e / NB : e % NB, b = rowcont ? e % NB : e / NB;
     r[u] = (a < rows && b < cols) ? __ldcg(v.p + (int64_t)a * v.rs + (int64_t)b * v.cs) : T(0);
   }
 }
-template <int NC, typename T>
-__device__ __forceinline__ void store_regs(T* s, const T (&r)[Chunk<NC>::EPT], ViewT<T> v) {
+template <typename T>
+__device__ __forceinline__ void store_regs(T* s, const T (&r)[EPT], ViewT<T> v) {
   const bool rowcont = (v.cs == 1 || v.cs == -1) && !(v.rs == 1 || v.rs == -1);
 #pragma unroll
-  for (int u = 0; u < Chunk<NC>::EPT; ++u) {
+  for (int u = 0; u < EPT; ++u) {
     const int e = threadIdx.x + 256 * u;
-    const int a = rowcont ? e / NC : e % NB, b = rowcont ? e % NC : e / NB;
-    s[a * Chunk<NC>::LDX + b] = r[u];
+    const int a = rowcont ? e / NB : e % NB, b = rowcont ? e % NB : e / NB;
+    s[a * LDX + b] = r[u];
   }
 }
 // 64 x 64 column-major workspace tile -> element (a, b) at s[b * LDL + a].
@@ -151,56 +131,21 @@ __device__ __forceinline__ void lds4(const double* p, double (&v)[4]) {
   const double2 y = reinterpret_cast<const double2*>(p)[1];
   v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
 }
-// acc (+)= sign * A(64 x 64, k-major, stride LDL) * X(64 x NC, row stride LDX)
-// on the thread's TR x TC register tile (rows tr*TR.., columns tc*TC..).
-// 64 columns: per k one 16-byte read of A's column and one of X's row feed 16
-// FMAs.  8 columns: the k range is split over four groups of 64 threads
-// (thread = row), whose partial sums meet in P (4 x 8 rows of LDP) in group
-// order;
-// the call contains two block barriers, so every thread of the CTA makes it.
-template <bool kSub, int NC, typename T>
-__device__ __forceinline__ void tile_mma(T (&acc)[Chunk<NC>::TR][Chunk<NC>::TC], const T* A,
-                                         const T* X, int tr, int tc, T* P) {
-  constexpr int TR = Chunk<NC>::TR, TC = Chunk<NC>::TC, LX = Chunk<NC>::LDX;
-  if constexpr (NC == 64) {
+// acc (+)= sign * A(64 x 64, k-major, stride LDL) * X(64 x 64, row stride LDX)
+// on the thread's 4 x 4 register tile (rows 4 tr.., columns 4 tc..): per k one
+// 16-byte read of A's column and one of X's row feed 16 FMAs.
+template <bool kSub, typename T>
+__device__ __forceinline__ void tile_mma(T (&acc)[4][4], const T* A, const T* X, int tr, int tc) {
 #pragma unroll 8
-    for (int k = 0; k < NB; ++k) {
-      T a[4], x[4];
-      lds4(A + k * LDL + tr * 4, a);
-      lds4(X + k * LX + tc * 4, x);
+  for (int k = 0; k < NB; ++k) {
+    T a[4], x[4];
+    lds4(A + k * LDL + tr * 4, a);
+    lds4(X + k * LDX + tc * 4, x);
 #pragma unroll
-      for (int p = 0; p < TR; ++p)
+    for (int p = 0; p < 4; ++p)
 #pragma unroll
-        for (int q = 0; q < TC; ++q)
-          acc[p][q] = kSub ? fma(-a[p], x[q], acc[p][q]) : fma(a[p], x[q], acc[p][q]);
-    }
-  } else {
-    static_assert(NC == 8 && TC == 1, "8-column chunk layout");
-    const int r = threadIdx.x % NB, g = threadIdx.x / NB;
-    T part[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) part[q] = T(0);
-#pragma unroll 4
-    for (int kk = 0; kk < NB / 4; ++kk) {
-      const int k = g * (NB / 4) + kk;
-      const T a = A[k * LDL + r];
-      T x[8];
-      lds4(X + k * LX, *reinterpret_cast<T(*)[4]>(x));
-      lds4(X + k * LX + 4, *reinterpret_cast<T(*)[4]>(x + 4));
-#pragma unroll
-      for (int q = 0; q < 8; ++q) part[q] = fma(a, x[q], part[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) P[(g * 8 + q) * LDP + r] = part[q];
-    __syncthreads();
-#pragma unroll
-    for (int p = 0; p < TR; ++p) {
-      const int row = tr * TR + p;
-      const T v = ((P[tc * LDP + row] + P[(8 + tc) * LDP + row]) + P[(16 + tc) * LDP + row]) +
-                  P[(24 + tc) * LDP + row];
-      acc[p][0] = kSub ? acc[p][0] - v : acc[p][0] + v;
-    }
-    __syncthreads();
+      for (int q = 0; q < 4; ++q)
+        acc[p][q] = kSub ? fma(-a[p], x[q], acc[p][q]) : fma(a[p], x[q], acc[p][q]);
   }
 }
 
@@ -222,50 +167,46 @@ __device__ __forceinline__ int wait_flag(const int* f, int* err) {
 // sync layout: sync[0] = ticket counter, sync[1 + b*nchunk + c] = flag of
 // block row b, chunk c (0 = not ready, 1 = ready, -1 = poisoned).
 // All zero at launch.  W: kInvStride elements per block row ([W_j | M_j]).
-// FP32: up to two CTAs per SM (104 KB of shared memory each; launches of at
-// most two chunks ask for one CTA per SM); FP64: one (204 KiB).
-template <typename T, int NC = 64>
+// FP32: up to two CTAs per SM (104 KB of shared memory each); FP64: one (204 KiB).
+template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1)
     trsm_wave(ViewT<T> L, int n, ViewT<T> B, int m, T alpha, const T* __restrict__ W,
               int* sync, int* err, const int* abort_flag) {
-  constexpr int TR = Chunk<NC>::TR, TC = Chunk<NC>::TC, EPT = Chunk<NC>::EPT;
-  constexpr int LX = Chunk<NC>::LDX;
   extern __shared__ __align__(16) unsigned char dyn_tsv_raw[];
   T* Ls0 = reinterpret_cast<T*>(dyn_tsv_raw);
   T* Ls1 = Ls0 + NB * LDL;
   T* Ws = Ls1 + NB * LDL;
   T* Xs0 = Ws + NB * LDL;
-  T* Xs1 = Xs0 + NB * LX;
-  T* Ts = Xs1 + NB * LX;
-  T* Ps = Ts + NB * LX;  // k-split partial sums (8-column chunks)
+  T* Xs1 = Xs0 + NB * LDX;
+  T* Ts = Xs1 + NB * LDX;
   __shared__ int sh_ticket, sh_state, sh_ready[2], sh_last;
   if (abort_flag && *abort_flag != INT_MAX) return;
   const int tid = threadIdx.x;
-  const int nchunk = (m + NC - 1) / NC;
+  const int nchunk = (m + NB - 1) / NB;
   if (tid == 0) sh_ticket = atomicAdd(sync, 1);
   __syncthreads();
   const int t = sh_ticket;
   const int j = t / nchunk, c = t % nchunk;
-  const int r0 = j * NB, c0 = c * NC;
-  const int rows = min(NB, n - r0), cols = min(NC, m - c0);
-  const int tr = tid / (NC / TC), tc = tid % (NC / TC);  // TR x TC register tile
+  const int r0 = j * NB, c0 = c * NB;
+  const int rows = min(NB, n - r0), cols = min(NB, m - c0);
+  const int tr = tid / 16, tc = tid % 16;  // 4 x 4 register tile
   int* flags = sync + 1;
   const ViewT<T> Bt = sub(B, r0, c0);
   const T* Wj = W + (int64_t)j * kInvStride;
   auto xview = [&](int i) { return sub(B, (int64_t)i * NB, c0); };
   auto lview = [&](int i) { return sub(L, r0, (int64_t)i * NB); };
 
-  T acc[TR][TC];
+  T acc[4][4];
 #pragma unroll
-  for (int a = 0; a < TR; ++a)
+  for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int b = 0; b < TC; ++b) acc[a][b] = T(0);
+    for (int b = 0; b < 4; ++b) acc[a][b] = T(0);
 
   // Loads that depend on no other CTA: W_j, B_jc, the first L tile.
   T xr[EPT];
   load_ws(Ws, Wj);
-  load_regs<NC>(xr, Bt, rows, cols);
-  store_regs<NC>(Ts, xr, Bt);
+  load_regs(xr, Bt, rows, cols);
+  store_regs(Ts, xr, Bt);
   const int iend = j - 1;  // products in the loop: i < iend
   bool poisoned = false;
   if (iend > 0) {
@@ -275,8 +216,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1)
     if (sh_state < 0) {
       poisoned = true;
     } else {
-      load_regs<NC>(xr, xview(0), NB, cols);
-      store_regs<NC>(Xs0, xr, xview(0));
+      load_regs(xr, xview(0), NB, cols);
+      store_regs(Xs0, xr, xview(0));
     }
   }
   cp_commit();
@@ -293,8 +234,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1)
     const bool ready = more && sh_ready[i & 1] > 0;
     if (more) load_tile<LDL>(Ln, lview(i + 1), rows, NB);
     cp_commit();
-    if (ready) load_regs<NC>(xr, xview(i + 1), NB, cols);
-    tile_mma<false, NC>(acc, Lb, Xb, tr, tc, Ps);
+    if (ready) load_regs(xr, xview(i + 1), NB, cols);
+    tile_mma<false>(acc, Lb, Xb, tr, tc);
     if (more) {
       if (!ready) {
         if (tid == 0) sh_state = wait_flag(&flags[(i + 1) * nchunk + c], err);
@@ -303,9 +244,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1)
           poisoned = true;
           break;
         }
-        load_regs<NC>(xr, xview(i + 1), NB, cols);
+        load_regs(xr, xview(i + 1), NB, cols);
       }
-      store_regs<NC>(Xn, xr, xview(i + 1));
+      store_regs(Xn, xr, xview(i + 1));
     }
   }
   if (poisoned) {
@@ -323,17 +264,17 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1)
   const bool ready = j > 0 && sh_last > 0;
   if (j > 0) load_ws(Ls0, Wj + NB * NB);
   cp_commit();
-  if (ready) load_regs<NC>(xr, xview(j - 1), NB, cols);
+  if (ready) load_regs(xr, xview(j - 1), NB, cols);
 #pragma unroll
-  for (int p = 0; p < TR; ++p)
+  for (int p = 0; p < 4; ++p)
 #pragma unroll
-    for (int q = 0; q < TC; ++q) {
-      T* tp = Ts + (tr * TR + p) * LX + tc * TC + q;
+    for (int q = 0; q < 4; ++q) {
+      T* tp = Ts + (tr * 4 + p) * LDX + tc * 4 + q;
       *tp = fma(alpha, *tp, -acc[p][q]);
       acc[p][q] = T(0);
     }
   __syncthreads();
-  tile_mma<false, NC>(acc, Ws, Ts, tr, tc, Ps);
+  tile_mma<false>(acc, Ws, Ts, tr, tc);
   if (j > 0) {
     if (!ready) {
       if (tid == 0) sh_state = wait_flag(&flags[(j - 1) * nchunk + c], err);
@@ -344,27 +285,27 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1)
         if (tid == 0) st_release(&flags[j * nchunk + c], -1);
         return;
       }
-      load_regs<NC>(xr, xview(j - 1), NB, cols);
+      load_regs(xr, xview(j - 1), NB, cols);
     }
-    store_regs<NC>(Xs0, xr, xview(j - 1));
+    store_regs(Xs0, xr, xview(j - 1));
     cp_wait_all();
     __syncthreads();
-    tile_mma<true, NC>(acc, Ls0, Xs0, tr, tc, Ps);  // X_j = Y - M_j X_{j-1}
+    tile_mma<true>(acc, Ls0, Xs0, tr, tc);  // X_j = Y - M_j X_{j-1}
   }
   // X_jc -> B through shared memory (Xs1 is free here), so that the global
   // stores run along B's contiguous dimension like the loads of load_regs.
 #pragma unroll
-  for (int p = 0; p < TR; ++p)
+  for (int p = 0; p < 4; ++p)
 #pragma unroll
-    for (int q = 0; q < TC; ++q) Xs1[(tr * TR + p) * LX + tc * TC + q] = acc[p][q];
+    for (int q = 0; q < 4; ++q) Xs1[(tr * 4 + p) * LDX + tc * 4 + q] = acc[p][q];
   __syncthreads();
   {
     const bool rowcont = (Bt.cs == 1 || Bt.cs == -1) && !(Bt.rs == 1 || Bt.rs == -1);
 #pragma unroll
     for (int u = 0; u < EPT; ++u) {
       const int e = tid + 256 * u;
-      const int a = rowcont ? e / NC : e % NB, b = rowcont ? e % NC : e / NB;
-      if (a < rows && b < cols) Bt.p[(int64_t)a * Bt.rs + (int64_t)b * Bt.cs] = Xs1[a * LX + b];
+      const int a = rowcont ? e / NB : e % NB, b = rowcont ? e % NB : e / NB;
+      if (a < rows && b < cols) Bt.p[(int64_t)a * Bt.rs + (int64_t)b * Bt.cs] = Xs1[a * LDX + b];
     }
   }
   // The block's stores are ordered before thread 0's release by the
