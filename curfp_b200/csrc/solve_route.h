@@ -49,12 +49,14 @@ enum SolveKernel {
 // 16384 columns: 64 a chunk 70 / 88 / 208 us, tiles 77 / 79 / 148).
 // FP64: 8 columns a chunk, up to 2048 (block row, chunk) pairs and 128 columns,
 // then 64 a chunk (order 16384, 65 / 100 / 128 columns: 7.1 / 8.8 / 10.7 ms
-// against 8.7 / 8.8 / 8.8; order 32768, 33 / 64: 14.4 / 19.5 against 17.2 /
-// 17.5).
+// against 8.7 / 8.8 / 8.8; order 32768, 33 / 64 / 100: 14.4 / 19.5 / 32.6 against
+// 17.2 / 17.5 / 27.7), unless that leaves nearly half of the columns empty (order
+// 32768, 65: 26.2 against 27.5).
 inline SolveKernel solve_kernel(bool fp32, int n, int m) {
   const int64_t nblk = (n + kTrsmLeaf - 1) / kTrsmLeaf;
   if (!fp32)
-    return m <= 128 && nblk * ((m + 7) / 8) < 2048 ? SOLVE_CHAIN8 : SOLVE_WAVE64;
+    return (m <= 128 && nblk * ((m + 7) / 8) < 2048) || (m > 64 && m <= 72) ? SOLVE_CHAIN8
+                                                                            : SOLVE_WAVE64;
   if (m == 1) return SOLVE_CHAIN1;
   if (m >= 4096) return SOLVE_TILES;
   if (m > 448 || (m >= 256 && (nblk <= 4 || n > 8192))) return SOLVE_WAVE64;

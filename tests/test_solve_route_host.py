@@ -38,7 +38,8 @@ def test_fp32_kernels(hostsim, n, m, kernel):
 
 
 @pytest.mark.parametrize("n,m,kernel", [(64, 1, CHAIN8), (8192, 120, CHAIN8), (8192, 121, WAVE64),
-                                        (16384, 56, CHAIN8), (16384, 57, WAVE64),
+                                        (16384, 56, CHAIN8), (16384, 57, WAVE64), (16384, 64, WAVE64),
+                                        (16384, 65, CHAIN8), (16384, 72, CHAIN8), (16384, 73, WAVE64),
                                         (64, 128, CHAIN8), (64, 129, WAVE64), (512, 4096, WAVE64)])
 def test_fp64_kernels(hostsim, n, m, kernel):
     assert route(hostsim, n, m, fp32=0, math=0)[2] == kernel
