@@ -179,6 +179,7 @@ curfpStatus_t curfpDestroy(curfpHandle_t handle) {
     cudaStreamSynchronize(handle->copy_stream);
     cudaStreamDestroy(handle->copy_stream);
   }
+  if (handle->ev_scratch) cudaEventDestroy(handle->ev_scratch);
   if (handle->ev_start) cudaEventDestroy(handle->ev_start);
   if (handle->ev_rest) cudaEventDestroy(handle->ev_rest);
   if (handle->pool) cudaMemPoolDestroy(handle->pool);
@@ -231,6 +232,7 @@ curfpStatus_t curfpDiagWaitTimeout(curfpHandle_t handle, int* err_code) {
 // src/curfp_handle.cpp:37-43
 curfpStatus_t curfpSetStream(curfpHandle_t handle, cudaStream_t stream) {
   if (!handle) return CURFP_STATUS_NOT_INITIALIZED;
+  rfp::order_after_scratch(handle, stream);
   handle->stream = stream;
   return CURFP_STATUS_SUCCESS;
 }
@@ -578,6 +580,7 @@ curfpStatus_t curfpSsfmmAcc64(curfpHandle_t handle, curfpOperation_t transr,
   if (n == 0 || nrhs == 0) return CURFP_STATUS_SUCCESS;
   if (ldx < n || ldy < n) return CURFP_STATUS_INVALID_VALUE;
   Geometry g = rfp::geometry(n, transr == CURFP_OP_T, uplo == CURFP_FILL_MODE_LOWER);
+  rfp::ScratchScope scratch(handle);
   return status_of(symm_launch(handle, g, A, X, ldx, Y, ldy, nrhs, *alpha, *beta));
 }
 
@@ -635,6 +638,7 @@ static curfpStatus_t sfmv_impl(curfpHandle_t handle, curfpOperation_t transr,
     return status_of(rfp::plan::rfp_symm(ex, tr, lower, n, arf, X, Y, 1, *alpha, *beta));
   }
   const Geometry g = rfp::geometry(n, tr, lower);
+  rfp::ScratchScope scratch(handle);
   if constexpr (sizeof(T) == 4) {
     rfp::ksymv2::Args a{};
     const int64_t total = rfp::ksymv2::plan(g, &a);

@@ -42,6 +42,12 @@ struct curfpContext {
   size_t wst_bytes = 0;
   void* wsg = nullptr;     // adjoint scratch (solve adjoint n x 2nrhs, NLL gradient)
   size_t wsg_bytes = 0;
+  // Workspaces are one set per handle, whatever its stream: an entry point that
+  // returns with work on them still in flight records ev_scratch behind it, and
+  // the stream that the handle is bound to next waits for it.
+  bool scratch_used = false;     // a workspace was handed out since the last record or synchronisation
+  bool scratch_pending = false;  // ev_scratch is recorded
+  cudaEvent_t ev_scratch = nullptr;
   cudaStream_t copy_stream = nullptr;  // host-input factorization: the overlapped copy
   cudaEvent_t ev_start = nullptr, ev_rest = nullptr;
 };
@@ -66,13 +72,28 @@ constexpr int kCholRfpRows = 4096;
 constexpr int kTriRows = 2048;
 constexpr int kLeafRows = 1024;
 
+// An entry point's use of the workspaces (exec_cuda.cu): records ev_scratch at
+// its end unless it synchronised after the last use.
+class ScratchScope {
+ public:
+  explicit ScratchScope(curfpContext* ctx) : ctx_(ctx) {}
+  ScratchScope(const ScratchScope&) = delete;
+  ScratchScope& operator=(const ScratchScope&) = delete;
+  ~ScratchScope();
+
+ private:
+  curfpContext* ctx_;
+};
+// Orders `stream` after the recorded use of the workspaces.
+void order_after_scratch(curfpContext* ctx, cudaStream_t stream);
+
 // The CUDA executor for FP32 (SIMT and split-BF16 tensor-core contractions)
 // and FP64 (SIMT DFMA) element types.
 template <typename T>
 class CudaExecT : public ExecT<T> {
  public:
   explicit CudaExecT(curfpContext* ctx, const int* abort_flag = nullptr)
-      : ctx_(ctx), abort_(abort_flag) {}
+      : ctx_(ctx), abort_(abort_flag), scratch_(ctx) {}
   int gemm(const GemmProbT<T>* p, int count) override;
   int potrf_tile(ViewT<T> L, int n, int info_base) override;
   int potrf_tile_rows() const override { return kCholRows; }
@@ -108,6 +129,9 @@ class CudaExecT : public ExecT<T> {
  protected:
   curfpContext* ctx_;
   const int* abort_;
+
+ private:
+  ScratchScope scratch_;
 };
 using CudaExec = CudaExecT<float>;
 using CudaExecD = CudaExecT<double>;

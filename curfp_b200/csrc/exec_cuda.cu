@@ -21,6 +21,7 @@
 namespace rfp {
 
 void* grow_buffer(curfpContext* ctx, void** buf, size_t* cur, size_t bytes) {
+  ctx->scratch_used = true;
   if (*buf && *cur >= bytes) return *buf;
   if (*buf) {
     cudaFreeAsync(*buf, ctx->stream);
@@ -43,6 +44,41 @@ void* grow_buffer(curfpContext* ctx, void** buf, size_t* cur, size_t bytes) {
   *buf = p;
   *cur = want;
   return p;
+}
+
+namespace {
+// Work captured into a graph neither records nor waits: the event belongs to
+// what has been launched, and a wait for it would break the capture.  (An error:
+// the legacy stream while another one captures.)
+bool capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus status;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return status != cudaStreamCaptureStatusNone;
+}
+}  // namespace
+
+ScratchScope::~ScratchScope() {
+  if (!ctx_->scratch_used) return;
+  ctx_->scratch_used = false;
+  if (capturing(ctx_->stream)) return;
+  if ((ctx_->ev_scratch ||
+       cudaEventCreateWithFlags(&ctx_->ev_scratch, cudaEventDisableTiming) == cudaSuccess) &&
+      cudaEventRecord(ctx_->ev_scratch, ctx_->stream) == cudaSuccess) {
+    ctx_->scratch_pending = true;
+    return;
+  }
+  cudaGetLastError();
+  cudaStreamSynchronize(ctx_->stream);
+}
+
+void order_after_scratch(curfpContext* ctx, cudaStream_t stream) {
+  if (!ctx->scratch_pending || capturing(stream)) return;
+  if (cudaStreamWaitEvent(stream, ctx->ev_scratch, 0) == cudaSuccess) return;
+  cudaGetLastError();
+  cudaEventSynchronize(ctx->ev_scratch);
 }
 
 template <typename T>

@@ -43,6 +43,7 @@ inline bool read(curfpContext* h, int* info, int* err) {
     cudaGetLastError();
     return false;
   }
+  h->scratch_used = h->scratch_pending = false;
   *info = w[0];
   *err = w[1];
   return true;

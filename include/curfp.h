@@ -77,6 +77,8 @@ typedef struct curfpContext *curfpHandle_t;
  * (src/curfp_handle.cpp:4-51). */
 curfpStatus_t curfpCreate(curfpHandle_t *handle);
 curfpStatus_t curfpDestroy(curfpHandle_t handle);
+/* The handle's workspaces are one set: what the new stream gets waits for the
+ * calls on the old one that still use them (except inside a stream capture). */
 curfpStatus_t curfpSetStream(curfpHandle_t handle, cudaStream_t stream);
 curfpStatus_t curfpGetStream(curfpHandle_t handle, cudaStream_t *stream);
 
