@@ -147,7 +147,7 @@ int launch_gemm(const GemmProbT<T>* p, int count, const int* abort_flag,
   if (splits > 1) {
     b.part = static_cast<T*>(grow_buffer(ctx, &ctx->wst, &ctx->wst_bytes,
                                          (size_t)splits * tiles * BM * BN * sizeof(T)));
-    if (!b.part) return 2;
+    if (!b.part) splits = 1;  // no memory: one range, no scratch
   }
   ProfScope ps(ctx->prof, st, K_SGEMM, flops, 0);
   ps.shape(b.p[0].m, b.p[0].n, b.p[0].k + b.p[0].k2, tiles);
@@ -186,7 +186,10 @@ int launch_skinny(const GemmProbT<T>& g0, const int* abort_flag, curfpContext* c
   if (splits > 1) {
     a.part = static_cast<T*>(grow_buffer(ctx, &ctx->wst, &ctx->wst_bytes,
                                          (size_t)splits * g.n * g.m * sizeof(T)));
-    if (!a.part) return 2;
+    if (!a.part) {  // no memory: one range, no scratch
+      splits = 1;
+      a.kseg = g.k;
+    }
   }
   const dim3 grid((g.m + 31) / 32, splits);
   cudaStream_t st = ctx->stream;
@@ -744,22 +747,25 @@ int launch_solve_tiles(curfpContext* ctx, const int* abort_flag, ViewT<T> L, int
 }
 }  // namespace
 
-// The kernels' choice: solve_route.h.
+// The kernels' choice: solve_route.h.  The wavefront solve needs the least
+// scratch (its flags); it stands in where another kernel's does not fit (rc 2:
+// nothing was launched).
 template <typename T>
 int CudaExecT<T>::trsm_wave(ViewT<T> L, int n, ViewT<T> B, int m, T alpha, const T* W) {
   if (n <= 0 || m <= 0) return 0;
   const SolveKernel kernel = solve_kernel(sizeof(T) == 4, n, m);
+  int rc = 2;
   if constexpr (sizeof(T) == 4) {
     switch (kernel) {
-      case SOLVE_CHAIN1: return launch_chain1(ctx_, abort_, L, n, B, alpha, W);
-      case SOLVE_CHAIN16: return launch_chain<T, 16>(ctx_, abort_, L, n, B, m, alpha, W);
-      case SOLVE_CHAIN32: return launch_chain<T, 32>(ctx_, abort_, L, n, B, m, alpha, W);
-      case SOLVE_TILES: return launch_solve_tiles<T>(ctx_, abort_, L, n, B, m, alpha, W);
+      case SOLVE_CHAIN1: rc = launch_chain1(ctx_, abort_, L, n, B, alpha, W); break;
+      case SOLVE_CHAIN16: rc = launch_chain<T, 16>(ctx_, abort_, L, n, B, m, alpha, W); break;
+      case SOLVE_CHAIN32: rc = launch_chain<T, 32>(ctx_, abort_, L, n, B, m, alpha, W); break;
+      case SOLVE_TILES: rc = launch_solve_tiles<T>(ctx_, abort_, L, n, B, m, alpha, W); break;
       default: break;
     }
   }
-  if (kernel == SOLVE_CHAIN8) return launch_chain<T, 8>(ctx_, abort_, L, n, B, m, alpha, W);
-  return launch_wave<T>(ctx_, abort_, L, n, B, m, alpha, W);
+  if (kernel == SOLVE_CHAIN8) rc = launch_chain<T, 8>(ctx_, abort_, L, n, B, m, alpha, W);
+  return rc == 2 ? launch_wave<T>(ctx_, abort_, L, n, B, m, alpha, W) : rc;
 }
 
 template class CudaExecT<float>;

@@ -37,6 +37,11 @@ inline GemmProbT<T> gemm_prob(ViewT<T> A, ViewT<T> B, ViewT<T> C, int m, int n, 
   return p;
 }
 
+// A block operation that found no scratch has done nothing: the recursion goes
+// on with smaller blocks, which need less, down to `least` rows.
+constexpr int kNoMemory = 2;
+inline bool smaller(int rc, int n, int least) { return rc == kNoMemory && n > least; }
+
 template <typename T>
 int trsm_rec(ExecT<T>& ex, ViewT<T> L, int n, ViewT<T> B, int m, Scalar<T> alpha,
              const T* W, int blk0, int math) {
@@ -116,7 +121,8 @@ int trmm_lln(ExecT<T>& ex, ViewT<T> L, int n, ViewT<T> B, int m, Scalar<T> alpha
     GemmProbT<T> p = gemm_prob(L, B, B, n, m, n, alpha, 0.0f, 0);
     p.a_tri = 1;
     p.inplace = 1;
-    return ex.gemm(&p, 1);
+    const int rc = ex.gemm(&p, 1);
+    if (!smaller(rc, n, kTriTile)) return rc;
   }
   int n1 = split(n, kTriTile), n2 = n - n1;
   int rc = trmm_lln(ex, sub(L, n1, n1), n2, sub(B, n1, 0), m, alpha, math);
@@ -146,13 +152,16 @@ template <typename T>
 int potrf_lower(ExecT<T>& ex, ViewT<T> A, int n, int info_base, int math) {
   if (n <= 0) return 0;
   const int tile = ex.potrf_tile_rows();
-  if (n <= tile) return ex.potrf_tile(A, n, info_base);
+  int rc;
+  if (n <= tile) {
+    rc = ex.potrf_tile(A, n, info_base);
+    if (!smaller(rc, n, kPotrfTile)) return rc;
+  }
   int n1 = split(n, kPotrfTile), n2 = n - n1;
   ViewT<T> A21 = sub(A, n1, 0);
-  int rc;
-  if (ex.has_panel(n1, n2)) {
-    if ((rc = ex.potrf_panel(A, A21, n1, n2, info_base))) return rc;
-  } else {
+  rc = ex.has_panel(n1, n2) ? ex.potrf_panel(A, A21, n1, n2, info_base) : kNoMemory;
+  if (rc && rc != kNoMemory) return rc;
+  if (rc) {
     if ((rc = potrf_lower(ex, A, n1, info_base, math))) return rc;
     // A21 := A21 L11^{-T}   <=>   L11 A21^T = A21^T
     if ((rc = trsm_lln(ex, A, n1, tr(A21), n2, 1.0f, math))) return rc;
@@ -166,10 +175,13 @@ int potrf_lower(ExecT<T>& ex, ViewT<T> A, int n, int info_base, int math) {
 template <typename T>
 int trtri_lower(ExecT<T>& ex, ViewT<T> L, int n, int math) {
   if (n <= 0) return 0;
-  if (n <= ex.trtri_rows()) return ex.trtri_block(L, n);
+  int rc;
+  if (n <= ex.trtri_rows()) {
+    rc = ex.trtri_block(L, n);
+    if (!smaller(rc, n, kTriTile)) return rc;
+  }
   int n1 = split(n, kTriTile), n2 = n - n1;
-  int rc = trtri_lower(ex, L, n1, math);
-  if (rc) return rc;
+  if ((rc = trtri_lower(ex, L, n1, math))) return rc;
   if ((rc = trtri_lower(ex, sub(L, n1, n1), n2, math))) return rc;
   ViewT<T> L21 = sub(L, n1, 0);
   // L21 := -inv(L22) L21 inv(L11)
@@ -180,11 +192,14 @@ int trtri_lower(ExecT<T>& ex, ViewT<T> L, int n, int math) {
 template <typename T>
 int lauum_lower(ExecT<T>& ex, ViewT<T> L, int n, int math) {
   if (n <= 0) return 0;
-  if (n <= ex.lauum_rows()) return ex.lauum_block(L, n);
+  int rc;
+  if (n <= ex.lauum_rows()) {
+    rc = ex.lauum_block(L, n);
+    if (!smaller(rc, n, kTriTile)) return rc;
+  }
   int n1 = split(n, kTriTile), n2 = n - n1;
   ViewT<T> L21 = sub(L, n1, 0);
-  int rc = lauum_lower(ex, L, n1, math);
-  if (rc) return rc;
+  if ((rc = lauum_lower(ex, L, n1, math))) return rc;
   // L11 += L21^T L21 (lower): a SYRK whose one operand is L21^T (n1 x n2)
   SharedTaskT<T> t{0, 0, n1, n1, L, 1.0f, 1.0f, 1};
   if ((rc = ex.gemm_shared(tr(L21), n1, n2, &t, 1, math))) return rc;
@@ -247,15 +262,20 @@ int spftrf(ExecT<T>& ex, int transr, int lower, int n, T* A, int math) {
   ViewT<T> V11 = block_view(A, g.b11), V21 = block_view(A, g.b21),
        V22 = block_view(A, g.b22);
   int rc = ex.potrf_blocks(V11, V21, V22, g.n1, g.n2);
-  if (rc != kNotSupported) return rc;
-  const bool panel = ex.has_panel(g.n1, g.n2);
-  if (!panel && (rc = potrf_lower(ex, V11, g.n1, 0, math))) return rc;
-  if ((rc = ex.after_first_block())) return rc;
-  if (g.n2 == 0) return 0;
+  if (rc != kNotSupported && rc != kNoMemory) return rc;
+  rc = kNoMemory;
+  if (ex.has_panel(g.n1, g.n2)) {
+    if ((rc = ex.after_first_block())) return rc;
+    rc = ex.potrf_panel(V11, V21, g.n1, g.n2, 0);
+    if (rc && rc != kNoMemory) return rc;
+  }
+  if (rc) {
+    if ((rc = potrf_lower(ex, V11, g.n1, 0, math))) return rc;
+    if ((rc = ex.after_first_block())) return rc;
+    if (g.n2 == 0) return 0;
+    if (g.n1 > 0 && (rc = trsm_lln(ex, V11, g.n1, tr(V21), g.n2, 1.0f, math))) return rc;
+  }
   if (g.n1 > 0) {
-    rc = panel ? ex.potrf_panel(V11, V21, g.n1, g.n2, 0)
-               : trsm_lln(ex, V11, g.n1, tr(V21), g.n2, 1.0f, math);
-    if (rc) return rc;
     SharedTaskT<T> t{0, 0, g.n2, g.n2, V22, -1.0f, 1.0f, 1};
     if ((rc = ex.gemm_shared(V21, g.n2, g.n1, &t, 1, math))) return rc;
   }
@@ -284,10 +304,10 @@ int spftrs(ExecT<T>& ex, int transr, int lower, int n, int nrhs, const T* A,
       at[i] = total;
       total += (size_t)inv_blocks(sz[i]) * kInvStride;
     }
-    T* w = ex.workspace(total);
-    if (!w) return 2;
-    if ((rc = ex.trtri_batch(L, sz, 4, w))) return rc;
-    for (int i = 0; i < 4; ++i) W[i] = w + at[i];
+    if (T* w = ex.workspace(total)) {  // else one triangle at a time
+      if ((rc = ex.trtri_batch(L, sz, 4, w))) return rc;
+      for (int i = 0; i < 4; ++i) W[i] = w + at[i];
+    }
   }
   // Forward: L Y = B.
   if ((rc = trsm_with<T>(ex, V11, g.n1, B1, nrhs, 1.0f, math, W[0]))) return rc;

@@ -192,9 +192,57 @@ class CpuExec : public Exec {
   int inplace_rows() const override { return 64; }
 };
 
+// An executor with block operations like the CUDA one's whose scratch never
+// fits: it refuses (rc 2, nothing done) every block above the recursions' last
+// sizes and a workspace for more than one triangle's records.
+class ScarceExec : public CpuExec {
+ public:
+  long refused = 0;
+  size_t ws_limit = SIZE_MAX;
+
+  int refuse() {
+    ++refused;
+    return 2;
+  }
+  int gemm(const GemmProb* p, int count) override {
+    if (count == 1 && p[0].inplace && p[0].m > 64) return refuse();
+    return CpuExec::gemm(p, count);
+  }
+  int potrf_tile_rows() const override { return 2048; }
+  int potrf_tile(View L, int n, int info_base) override {
+    return n > kPotrfTile ? refuse() : CpuExec::potrf_tile(L, n, info_base);
+  }
+  int potrf_blocks(View, View, View, int, int) override { return refuse(); }
+  bool has_panel(int n1, int n2) const override { return n1 > 0 && n2 > 0; }
+  int potrf_panel(View, View, int, int, int) override { return refuse(); }
+  int trtri_rows() const override { return 2048; }
+  int trtri_block(View L, int n) override { return n > kTriTile ? refuse() : trtri_tile(L, n); }
+  int lauum_rows() const override { return 1024; }
+  int lauum_block(View L, int n) override { return n > kTriTile ? refuse() : lauum_tile(L, n); }
+  int inplace_rows() const override { return 1024; }
+  bool batch_inverses() const override { return true; }
+  float* workspace(size_t count) override {
+    if (count <= ws_limit) return CpuExec::workspace(count);
+    ++refused;
+    return nullptr;
+  }
+};
+
 }  // namespace
 
 extern "C" {
+
+// spftrf, spftrs (4 columns of B) and spftri of one matrix on that executor;
+// returns the first rc, *refused counts the refusals.
+int hs_scarce(int transr, int lower, int n, float* A, float* B, long* refused) {
+  ScarceExec ex;
+  ex.ws_limit = (size_t)((n / 2 + kTrsmLeaf) / kTrsmLeaf) * kInvStride;
+  int rc = plan::spftrf(ex, transr, lower, n, A);
+  if (rc == 0) rc = plan::spftrs(ex, transr, lower, n, 4, A, B, n);
+  if (rc == 0) rc = plan::spftri(ex, transr, lower, n, A);
+  *refused = ex.refused;
+  return rc;
+}
 
 int hs_ssfrk(int transr, int lower, int trans, int n, int k, float alpha,
              const float* A, int lda, float beta, float* C, long* calls) {
