@@ -56,8 +56,12 @@ namespace rfp {
 
 // What the tile Cholesky (k_chol.cuh) takes in one launch: a diagonal block
 // of up to kCholRows, with up to kCholPanelRows rows below it, and a whole RFP
-// matrix of up to kCholRfpRows when its trailing update is too small for the
-// tensor cores (FP64: always).  Above, the recursion's larger products win.
+// matrix of up to kCholRfpRows (FP64), or up to where its trailing update is
+// large enough for the tensor cores (FP32, order 1300, in both math modes).  The
+// lines are where the launch has been proven, not where it stops winning.  One
+// launch against panel and update: FP32 n = 1300 311 / 358 us, 3000 651 / 716, 4096
+// 1097 / 1033 (FP32 mode 306 / 375, 651 / 853, 1098 / 1244); FP64 n = 5000 3.8 / 5.6
+// ms, 8192 12.4 / 14.2.
 constexpr int kCholRows = 2048;
 constexpr int kCholPanelRows = 2048;
 constexpr int kCholRfpRows = 4096;

@@ -9,6 +9,7 @@
 #include "func_attr.h"
 #include "gemm_route.h"
 #include "solve_route.h"
+#include "symv2_layout.h"
 #include "symv_layout.h"
 
 using namespace rfp;
@@ -51,6 +52,69 @@ int hs_symv_layout(int n, int64_t* out) {
   out[4] = col_over;
   out[5] = col_dup;
   out[6] = empty;
+  return 0;
+}
+
+// Enumerates the CTAs (g, s) of the ssfmv strips at order n the way the kernel
+// walks them.  out: [0] partial elements, [1] stored elements visited, [2]
+// visits outside the array or to an element already visited, [3] visits whose
+// y indices are not the element's row and column, [4] partial sums outside the
+// buffer or written twice, [5] steps not a multiple of the span.
+int hs_symv2_layout(int n, int transr, int lower, int64_t* out) {
+  const Geometry geo = geometry(n, transr, lower);
+  ksymv2::Args a{};
+  const int64_t total = ksymv2::plan(geo, &a);
+  const int64_t nt = (int64_t)n * (n + 1) / 2;
+  std::vector<int> row((size_t)nt, -1), col((size_t)nt, -1);  // logical indices of an offset
+  const BlockGeom* bg[3] = {&geo.b11, &geo.b21, &geo.b22};
+  const int pb[3] = {0, geo.n1, geo.n1}, qb[3] = {0, 0, geo.n1};
+  const int rows[3] = {geo.n1, geo.n2, geo.n2}, cols[3] = {geo.n1, geo.n1, geo.n2};
+  for (int i = 0; i < 3; ++i)
+    for (int p = 0; p < rows[i]; ++p)
+      for (int q = 0; q < cols[i]; ++q) {
+        if (i != 1 && q > p) continue;
+        const int64_t e = bg[i]->off + (int64_t)p * bg[i]->rs + (int64_t)q * bg[i]->cs;
+        row[(size_t)e] = pb[i] + p;
+        col[(size_t)e] = qb[i] + q;
+      }
+  std::vector<char> seen((size_t)nt, 0), part((size_t)total, 0);
+  int64_t visited = 0, bad = 0, wrong = 0, slots = 0, span = 0;
+  auto slot = [&](int64_t at) {
+    if (at < 0 || at >= total || part[(size_t)at]++) ++slots;
+  };
+  for (int bi = 0; bi < a.nblocks; ++bi) {
+    const ksymv2::Block& b = a.b[bi];
+    for (int g = 0; g < b.groups; ++g)
+      for (int s = 0; s < a.strips; ++s) {
+        int lo, hi;
+        ksymv2::l_range(b, g, lo, hi);
+        lo += s * a.span;
+        hi = hi < lo + a.span ? hi : lo + a.span;
+        if (lo >= hi) continue;
+        span += a.span % ksymv2::LT != 0;
+        for (int l = lo; l < hi; ++l) slot(b.lpart + (int64_t)g * b.ll + l);
+        for (int o = g * ksymv2::OG; o < b.lo && o < (g + 1) * ksymv2::OG; ++o) {
+          slot(b.opart + (int64_t)s * b.lo + o);
+          for (int l = lo; l < hi; ++l) {
+            if (!(b.tri == 0 || (b.tri == 1 ? l >= o : l <= o))) continue;
+            ++visited;
+            const int64_t e = b.off + l + o * b.so;
+            if (e < 0 || e >= nt || seen[(size_t)e]++) {
+              ++bad;
+              continue;
+            }
+            const int i = b.lbase + l, j = b.obase + o, r = row[(size_t)e], c = col[(size_t)e];
+            if (!((i == r && j == c) || (i == c && j == r))) ++wrong;
+          }
+        }
+      }
+  }
+  out[0] = total;
+  out[1] = visited;
+  out[2] = bad;
+  out[3] = wrong;
+  out[4] = slots;
+  out[5] = span;
   return 0;
 }
 
