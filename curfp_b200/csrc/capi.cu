@@ -373,7 +373,8 @@ curfpStatus_t curfpSpftrfEx(curfpHandle_t handle, curfpOperation_t transr,
 // stream (after everything already enqueued on the handle's stream) and the
 // factorization waits for it only after the first diagonal block, so that
 // for layouts where that block occupies its own part of the array (TRANSR =
-// T) the rest of the transfer overlaps its factorization.  With arf_orig the
+// T) the rest of the transfer overlaps its factorization; up to n = 4096 one
+// launch takes that block with others and the whole copy comes first.  With arf_orig the
 // host array is copied there and, region by region, on to arf (one
 // host-to-device transfer for both).
 curfpStatus_t curfpSpftrfFromHost(curfpHandle_t handle, curfpOperation_t transr,

@@ -72,6 +72,8 @@ constexpr int kAdjTile = 64;     // Cholesky-adjoint diagonal tiles
 constexpr int kTrsvMaxRhs = 512; // one-launch solves for at most this many RHS (solve_route.h)
 constexpr int kNotSupported = -1;
 
+// An operation that returns 2 has found no memory for its scratch and done
+// nothing; the planner then goes on with smaller blocks where it can.
 template <typename T>
 class ExecT {
  public:
@@ -102,9 +104,10 @@ class ExecT {
     (void)L; (void)A21; (void)n1; (void)n2; (void)info_base;
     return kNotSupported;
   }
-  // Called by the RFP factorization once the first diagonal block's work is
-  // enqueued and before any work that reads the other blocks: an executor
-  // may order that work after data it is still bringing in.
+  // Called by the RFP factorization before any work that reads the other
+  // blocks (once the first diagonal block's work is enqueued, where that is an
+  // operation of its own): an executor may order that work after data it is
+  // still bringing in.
   virtual int after_first_block() { return 0; }
   // Inverses of the diagonal nb x nb blocks of lower L (n x n): block b is
   // written to W + b*nb*nb, column-major with ld nb, zeros above the diagonal.

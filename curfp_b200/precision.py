@@ -75,8 +75,8 @@ def spftrf_from_host(C_host: torch.Tensor, C: torch.Tensor, C_orig: torch.Tensor
     """Copy the host RFP array C_host (CPU float32, contiguous; pinned for the
     copy to overlap) to the CUDA array C and factor it in place
     (curfpSpftrfFromHost); C_orig, if given, receives the unfactored matrix.
-    For transr = T the copy of the array's second part overlaps the
-    factorization of the first diagonal block."""
+    For transr = T and n > 4096 the copy of the array's second part overlaps
+    the factorization of the first diagonal block."""
     if C_host.device.type != "cpu" or C_host.dtype != torch.float32 or not C_host.is_contiguous():
         raise ValueError("C_host must be a contiguous float32 CPU tensor")
     _validate(C, "C")

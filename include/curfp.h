@@ -209,7 +209,9 @@ curfpStatus_t curfpSpftrfEx(curfpHandle_t handle, curfpOperation_t transr,
  * bus once.  The part of the array the first diagonal block touches is
  * copied first; the rest is copied on an internal stream and waited for only
  * after that block is factored, so for TRANSR = T (where that block occupies
- * its own half of the array) the transfer overlaps the factorization.
+ * its own half of the array) the transfer overlaps the factorization.  Up to
+ * n = 4096 one launch takes the first block together with the others, and
+ * the whole copy comes first.
  * Synchronises the handle's stream once to read info.  Not in the reference. */
 curfpStatus_t curfpSpftrfFromHost(curfpHandle_t handle, curfpOperation_t transr,
                                   curfpFillMode_t uplo, int n, const float *arf_host,
