@@ -9,15 +9,20 @@
 
 namespace rfp {
 
+// Elements of X from which the SMs are busy with one launch whatever its chain
+// of block rows does: the products' rate counts from here on.
+constexpr int64_t kSolveBusy = int64_t(9) << 18;
+
 // The whole triangle as one launch, or the recursion whose rectangle updates
 // are products on the tensor cores (math != 0): a launch does n^2 m operations
-// on the SIMT cores, so above 8192 rows the recursion wins from 128 columns on
-// (order 32768, 128 / 200 / 512 columns: 9.7 / 15.4 / 32.2 ms in one launch, 9.6 /
-// 10.8 / 17.2; order 65536: 35 / 57 / 119 and 28 / 33 / 50) and loses below (order
-// 65536, 64 / 100 columns: 24 / 45 and 27 / 47 ms; order 16384, 100 / 200 columns:
-// 3.7 / 4.5 and 4.3 / 4.0).
+// on the SIMT cores, so above 8192 rows and kSolveBusy elements the recursion
+// wins from 128 columns on (order 20000, 256 columns 7.6 ms in one launch, 7.5;
+// 24000, 200 9.2 / 7.5; 32768, 200 / 512 15.4 / 28 and 11.1 / 16.9; 65536, 128 / 512
+// 35 / 103 and 28 / 49).  Below it loses (17000, 128 / 256 3.4 / 5.8 and 4.8 / 6.1;
+// 24000, 128 5.9 / 6.7), and with fewer columns always (65536, 64 / 127 24 / 45 and
+// 27 / 48).
 inline bool solve_in_one_launch(int n, int m, int math) {
-  return m <= kTrsvMaxRhs && !(math && m >= 128 && n > 8192);
+  return m <= kTrsvMaxRhs && !(math && m >= 128 && n > 8192 && (int64_t)n * m >= kSolveBusy);
 }
 // Rows that the recursion leaves to one launch: small blocks, so that most of
 // the work is in the updates, but with few columns a launch of 512 rows is
@@ -38,15 +43,16 @@ enum SolveKernel {
 // allows, since the chain's step shrinks with the chunk while the products'
 // cost per column grows: 8 columns up to 256 (block row, chunk) pairs, 16 up to
 // 512, else 32 (8192 rows, 16 / 64 / 128 columns: 8 wide 190 / 510 / 970 us, 16
-// wide 262 / 390 / 690 us, 32 wide 400 / 420 / 600 us).  With more columns the
-// SMs are busy whatever the chain does, and 64 columns a chunk win: above 448
-// columns (order 2000, 400 / 512 columns: chain 535 / 642 us, here 611 / 534;
-// order 16384: 7.7 / 9.2 ms, here 7.6 / 8.2), and from 256 on in up to four block
-// rows, where half of each cluster is idle (order 250, 200 / 256 / 512: 167 / 183
-// / 233 us, here 163 / 164 / 163), and above 8192 rows (order 32768 in FP32 mode,
-// 200 / 320 / 400: 21.6 / 30.5 / 38.7 ms, here 22.9 / 29.5 / 37.4).  From 4096
-// columns on, 64 x 64 tiles with 8 x 8 register products (512 rows, 2048 / 4096 /
-// 16384 columns: 64 a chunk 70 / 88 / 208 us, tiles 77 / 79 / 148).
+// wide 262 / 390 / 690 us, 32 wide 400 / 420 / 600 us), and 32 from 256 columns on
+// where the triangle is one row of clusters (order 500, 256 / 480 columns: 8 wide
+// 248 / 299 us, 32 wide 199 / 198).  Chunks of 64 columns (k_trsv.cuh) win above
+// 480 columns, where 32-column chunks need another turn of clusters (order 500,
+// 480 / 481 / 512: 198 / 250 / 265 us, 64 wide 221 / 222 / 222; order 8192: 2.59 / 3.00
+// / 3.01 ms, 64 wide 2.78), and above 256 from kSolveBusy elements on (order 12000,
+// 440: 5.11 ms, 64 wide 4.62; order 16384, 384: 7.19 and 6.97; order 32768 in FP32
+// mode, 200 / 320 / 400: 21.6 / 30.5 / 38.7, 64 wide 22.9 / 29.5 / 37.4).  From 4096
+// columns on, 64 x 64 tiles with 8 x 8 register products (512 rows, 2048 / 4096 / 16384 columns: 64
+// wide 70 / 88 / 208 us, tiles 77 / 79 / 148).
 // FP64: 8 columns a chunk, up to 2048 (block row, chunk) pairs and 128 columns,
 // then 64 a chunk (order 16384, 65 / 100 / 128 columns: 7.1 / 8.8 / 10.7 ms
 // against 8.7 / 8.8 / 8.8; order 32768, 33 / 64 / 100: 14.4 / 19.5 / 32.6 against
@@ -59,8 +65,8 @@ inline SolveKernel solve_kernel(bool fp32, int n, int m) {
                                                                             : SOLVE_WAVE64;
   if (m == 1) return SOLVE_CHAIN1;
   if (m >= 4096) return SOLVE_TILES;
-  if (m > 448 || (m >= 256 && (nblk <= 4 || n > 8192))) return SOLVE_WAVE64;
-  if (nblk * ((m + 15) / 16) > 512) return SOLVE_CHAIN32;
+  if (m > 480 || (m > 256 && (int64_t)n * m >= kSolveBusy)) return SOLVE_WAVE64;
+  if (nblk * ((m + 15) / 16) > 512 || (m >= 256 && nblk <= 8)) return SOLVE_CHAIN32;
   return nblk * ((m + 7) / 8) > 256 ? SOLVE_CHAIN16 : SOLVE_CHAIN8;
 }
 

@@ -14,8 +14,9 @@ def route(hs, n, m, fp32=1, math=1):
     return list(out)
 
 
-@pytest.mark.parametrize("n,m,math,one", [(8192, 512, 1, 1), (8193, 512, 1, 0), (8193, 127, 1, 1),
-                                          (8193, 128, 1, 0), (65536, 64, 1, 1), (65536, 100, 1, 1),
+@pytest.mark.parametrize("n,m,math,one", [(8192, 512, 1, 1), (8193, 512, 1, 0), (8193, 128, 1, 1),
+                                          (9215, 256, 1, 1), (9216, 256, 1, 0), (18431, 128, 1, 1),
+                                          (18432, 128, 1, 0), (65536, 127, 1, 1),
                                           (65536, 128, 1, 0), (65536, 512, 0, 1), (100, 513, 0, 0),
                                           (100, 513, 1, 0), (1, 512, 1, 1)])
 def test_one_launch_or_recursion(hostsim, n, m, math, one):
@@ -26,12 +27,13 @@ def test_leaves(hostsim):
     assert route(hostsim, 9000, 512)[1] == 2048 and route(hostsim, 9000, 513)[1] == 512
 
 
-@pytest.mark.parametrize("n,m,kernel", [(64, 1, CHAIN1), (64, 2, CHAIN8), (256, 255, CHAIN8),
-                                        (256, 256, WAVE64), (257, 256, CHAIN8), (512, 449, WAVE64),
-                                        (512, 448, CHAIN16), (2048, 64, CHAIN8),
+@pytest.mark.parametrize("n,m,kernel", [(64, 1, CHAIN1), (64, 2, CHAIN8), (512, 255, CHAIN8),
+                                        (512, 256, CHAIN32), (513, 256, CHAIN16),
+                                        (512, 480, CHAIN32), (512, 481, WAVE64), (2048, 64, CHAIN8),
                                         (2048, 65, CHAIN16), (2048, 257, CHAIN32),
-                                        (8192, 448, CHAIN32), (8192, 449, WAVE64),
-                                        (8193, 255, CHAIN32), (8193, 256, WAVE64),
+                                        (4096, 480, CHAIN32), (4096, 481, WAVE64),
+                                        (8192, 287, CHAIN32), (8192, 288, WAVE64),
+                                        (16384, 256, CHAIN32), (16384, 257, WAVE64),
                                         (512, 4095, WAVE64), (512, 4096, TILES)])
 def test_fp32_kernels(hostsim, n, m, kernel):
     assert route(hostsim, n, m)[2] == kernel
