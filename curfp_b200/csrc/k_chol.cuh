@@ -526,7 +526,8 @@ __global__ void __launch_bounds__(threads<T>(), 1) chol_wave(const Args<T> g) {
   for (int h = 0; h < 2; ++h) {  // one copy of the code (instruction cache)
     if (warp == 0) {
       const int f = factor32(Ss + h * (32 * NB + 32), raw, 2 + 4 * h);
-      if (lane == 0 && f) sh_odd.x = 32 * h + f;
+      // (an infinite last pivot makes the padding's NaN: no failure)
+      if (lane == 0 && f && 32 * h + f <= sr) sh_odd.x = 32 * h + f;
     } else if (warp == 1) {
       const bool any = inverse32(Ws + h * (32 * LDW + 32), raw, 2 + 4 * h);
       if (lane == 0) sh_odd.y = any;
