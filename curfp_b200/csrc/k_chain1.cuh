@@ -56,14 +56,15 @@ __device__ __forceinline__ bool try_parity(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// late: a wait of this thread ran out before; it does not wait again.
-__device__ __forceinline__ void wait_parity(uint32_t bar, uint32_t parity, int* err, bool& late) {
-  if (late || try_parity(bar, parity)) return;
+// *late: a wait of this CTA ran out before; it does not wait again.
+__device__ __forceinline__ void wait_parity(uint32_t bar, uint32_t parity, int* err,
+                                            volatile int* late) {
+  if (try_parity(bar, parity) || *late) return;
   const uint64_t t0 = ktrsv::gtimer();
   while (!try_parity(bar, parity))
     if (ktrsv::gtimer() - t0 > ktrsv::WAIT_NS) {
       atomicExch(err, 5);
-      late = true;
+      *late = 1;
       return;
     }
 }
@@ -88,6 +89,7 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(THR, 1) chain1(cons
   __shared__ __align__(16) float Xr[XR][NB], Xin[CS - 1][NB], Ts[NB];
   __shared__ __align__(8) uint64_t full[XR], empty[XR], in[CS - 1];
   __shared__ int sh_ticket;
+  __shared__ volatile int sh_late;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = (int)kchain::cluster_rank();
   if (tid == 0) {
@@ -101,6 +103,7 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(THR, 1) chain1(cons
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(su32(&in[s])),
                    "r"((uint32_t)(NB * sizeof(float)))
                    : "memory");
+    sh_late = 0;
     if (rank == 0) sh_ticket = atomicAdd(g.sync, 1);
   }
   kchain::cluster_barrier();
@@ -111,7 +114,6 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(THR, 1) chain1(cons
                : "memory");
   q0 *= CS;
   const int j = q0 + rank;
-  bool late = false;
   if (j < g.nblk) {
     const int rows = min(NB, g.n - j * NB);
     const View Lj = sub(g.L, (int64_t)j * NB, 0);
@@ -160,17 +162,17 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(THR, 1) chain1(cons
         for (int u = 0; u < 4; ++u) {
           const int k = k0 + u;
           if (k >= nglob) break;
-          if (!(v[u] >> 32) && !late) {
+          if (!(v[u] >> 32) && !sh_late) {
             const uint64_t t0 = ktrsv::gtimer();
             while (!((v[u] = ld_word(p + (int64_t)k * NB)) >> 32))
               if (ktrsv::gtimer() - t0 > ktrsv::WAIT_NS) {
                 atomicExch(g.err, 5);
-                late = true;
+                sh_late = 1;
                 break;
               }
           }
           const int slot = k % XR, use = k / XR;
-          if (use > 0) wait_parity(su32(&empty[slot]), (use - 1) & 1, g.err, late);
+          if (use > 0) wait_parity(su32(&empty[slot]), (use - 1) & 1, g.err, &sh_late);
           Xr[slot][perm(e)] = __uint_as_float((unsigned)v[u]);
           arrive(su32(&full[slot]));
         }
@@ -191,10 +193,10 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(THR, 1) chain1(cons
         const float* x;
         const bool ring = k < nglob;
         if (ring) {
-          wait_parity(su32(&full[k % XR]), (k / XR) & 1, g.err, late);
+          wait_parity(su32(&full[k % XR]), (k / XR) & 1, g.err, &sh_late);
           x = Xr[k % XR];
         } else {
-          wait_parity(su32(&in[k - q0]), 0, g.err, late);
+          wait_parity(su32(&in[k - q0]), 0, g.err, &sh_late);
           x = Xin[k - q0];
         }
 #pragma unroll
@@ -267,10 +269,10 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(THR, 1) chain1(cons
   }
   // No CTA leaves while another may still write to its shared memory: every
   // send precedes the barrier, and every block sent here has been waited for.
-  // The barrier orders a send, not its arrival, so a thread that stopped
-  // waiting waits (bounded) for what was sent now.
+  // The barrier orders a send, not its arrival, so a CTA that stopped waiting
+  // waits (bounded) for what was sent now.
   kchain::cluster_barrier();
-  if (late && j < g.nblk) {
+  if (sh_late && j < g.nblk) {
     const uint64_t t0 = ktrsv::gtimer();
     for (int s = 0; s < rank; ++s)
       while (!try_parity(su32(&in[s]), 0) && ktrsv::gtimer() - t0 < 1000000ull) {}
